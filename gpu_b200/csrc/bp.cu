@@ -48,10 +48,10 @@ struct SharedTables {
 __device__ __forceinline__ SharedTables load_tables(const DevGeom& g, float* sp)
 {
     SharedTables t;
-    t.PX = sp;
+    t.RT = reinterpret_cast<float2*>(sp);   // first: 8-byte aligned whatever the plane counts
+    t.PX = sp + 2 * g.ZP;
     t.PY = t.PX + (g.M + 3);
     t.PZ = t.PY + (g.N + 3);
-    t.RT = reinterpret_cast<float2*>(t.PZ + ((g.Z + 3 + 1) & ~1));
     for (int q = threadIdx.x; q < g.M + 3; q += BP_THREADS) t.PX[q] = g.px[q];
     for (int q = threadIdx.x; q < g.N + 3; q += BP_THREADS) t.PY[q] = g.py[q];
     for (int q = threadIdx.x; q < g.Z + 3; q += BP_THREADS) t.PZ[q] = g.pz[q];
@@ -259,10 +259,10 @@ constexpr float ROW_EPS = 1.0f / 32.0f;   // margin of the alpha-range row estim
 __device__ __forceinline__ void walk_tables_addr(const DevGeom& g, float* sp, float*& PX, float*& PY, float*& PZ,
                                                  float2*& RT)
 {
-    PX = sp;
+    RT = reinterpret_cast<float2*>(sp);   // first: 8-byte aligned whatever the plane counts
+    PX = sp + 2 * g.ZP;
     PY = PX + (g.M + 3);
     PZ = PY + (g.N + 3);
-    RT = reinterpret_cast<float2*>(PZ + ((g.Z + 3 + 1) & ~1));
 }
 __device__ __forceinline__ void walk_tables(const DevGeom& g, float* sp, float*& PX, float*& PY, float*& PZ,
                                             float2*& RT)
