@@ -179,6 +179,18 @@ extern "C" ctr_status ctr_backproject(const ctr_geometry* geom, const float* sin
         if (!(flags & CTR_BP_ACCUMULATE)) CTR_CUDA_TRY(cudaMemsetAsync(vol, 0, g->nvox() * dtype_size(vdt), st));
         return CTR_OK;
     }
+    // The z-column gather reproduces the traversal of every scanner whose loop
+    // test is one comparison (no chord is cut short at the exit) with FP32
+    // entry; the other geometries and the masked form keep the general kernels.
+    if (!masked && g->dg.fast_exit && !g->dg.entry64 && g->dg.ct_style != 3) {
+        CTR_TRY(ensure_rays(g, adj_record_bytes(g->dg, std::min(batch, n))));
+        for (int c = 0; c < n; c += batch) {
+            const int cnt = std::min(batch, n - c);
+            CTR_TRY(launch_adjoint_cols(*g, sino + (size_t)c * P, v0 + c, cnt, g->d_rays, vol, vdt,
+                                        c > 0 || (flags & CTR_BP_ACCUMULATE), st));
+        }
+        return CTR_OK;
+    }
     CTR_TRY(ensure_rays(g, (size_t)P * batch * sizeof(AdjRay)));
     for (int c = 0; c < n; c += batch) {
         const int cnt = std::min(batch, n - c);

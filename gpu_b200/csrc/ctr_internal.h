@@ -205,6 +205,13 @@ struct __align__(16) AdjRay {
 ctr_status launch_ray_prep(const Geometry& g, const float* y, int view0, int nview, AdjRay* rays,
                            cudaStream_t st);
 
+// The matched adjoint as a z-column gather (zcol_adj.cu): views [view0,
+// view0 + nview) of y into vol.  ws: adj_record_bytes(g, nview) of scratch.
+// For fast_exit geometries with FP32 entry, the tetrahedron beam excepted.
+size_t adj_record_bytes(const DevGeom& g, int views);
+ctr_status launch_adjoint_cols(const Geometry& g, const float* y, int view0, int nview, void* ws, void* vol,
+                               ctr_dtype vdt, bool accumulate, cudaStream_t st);
+
 // slab SART: the slabs' partial sums [n_parts][P] added in slab order, the
 // SART correction of view `view` and the ray's d12 -> rays (slabs.cu); with
 // b == nullptr the weighted sums alone, as floats
