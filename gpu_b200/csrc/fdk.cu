@@ -5,12 +5,15 @@
 //   2. ramp filter.  The reference zero-pads each row to 2R, runs a cuFFT C2C,
 //      multiplies by |k|*F_step*0.5 and inverts (V63/FDK/FFT_1d_GPU.h:241-287),
 //      i.e. a linear convolution with h[n] = (1/2R) sum_k H[k] cos(pi k n / R),
-//      |n| < R.  Here h is computed once in FP64 on the host and the rows are
-//      convolved directly in a register-tiled Toeplitz kernel;
+//      |n| < R, h computed once in FP64 on the host.  Rows of up to
+//      kFftMost / 2 values are weighted and filtered in one kernel by an FFT in
+//      shared memory (k_ramp_fft); longer ones by a register-tiled Toeplitz
+//      product (k_fdk_weight, k_ramp);
 //   3. voxel-driven bilinear backprojection, kernel_FDK_reconstruction
 //      (V63/FDK/kernel_FDK.cu:16-62), with a batch of views per launch held in
 //      registers (each view's update is still applied with the reference's
 //      float/double steps, so the sum is the reference's to the bit).
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -93,7 +96,172 @@ k_ramp(const float* __restrict__ in, float* __restrict__ out, const float* __res
     }
 }
 
-static constexpr int FB_BX = 32, FB_BY = 4, FB_K = 4;
+// ---- weight and ramp of two detector rows by FFT
+//
+// The taps are real and even, so their spectrum is real: a row pair a + i b
+// stays a pair through FFT, product and inverse FFT, and no unpacking is
+// needed.  n = a power of two >= 2R - 1 points; Stockham passes of radix 8
+// (radix 4 or 2 last), 8 points a thread, exchanged through one padded
+// shared-memory buffer.  The first pass reads the rows (weighted on the way,
+// zero beyond R), the last inverse pass writes them.
+// 1024-point rows: 15 n log2 n = 0.34 MFLOP a pair instead of the Toeplitz
+// product's 4.2 M multiply-adds; bound by shared memory (7 exchanges).
+// 1024 views x 768 rows of 1024: 12.3 ms, weight included (Toeplitz 37.6 ms and
+// the weight pass 3.3 ms).
+static constexpr int kFftMost = 8192;   // 1024 threads, 147 KB of shared memory
+
+__device__ __forceinline__ int fft_pad(int i) { return i + (i >> 3); }
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ float2 cmul(float2 a, float2 b)
+{
+    return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
+}
+// i*a (inverse) or -i*a (forward)
+template <bool INV> __device__ __forceinline__ float2 crot(float2 a)
+{
+    return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+}
+template <bool INV> __device__ __forceinline__ void fft2(float2& a, float2& b)
+{
+    const float2 t = csub(a, b);
+    a = cadd(a, b);
+    b = t;
+}
+template <bool INV> __device__ __forceinline__ void fft4(float2* v)   // in order
+{
+    float2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]), c = cadd(v[1], v[3]), d = crot<INV>(csub(v[1], v[3]));
+    v[0] = cadd(a, c);
+    v[1] = cadd(b, d);
+    v[2] = csub(a, c);
+    v[3] = csub(b, d);
+}
+template <bool INV> __device__ __forceinline__ void fft8(float2* v)   // in order
+{
+    const float h = 0.70710678118654752440f;
+    float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+    fft4<INV>(e);
+    fft4<INV>(o);
+    const float2 w1 = INV ? make_float2(h, h) : make_float2(h, -h), w3 = INV ? make_float2(-h, h) : make_float2(-h, -h);
+    o[1] = cmul(o[1], w1);
+    o[2] = crot<INV>(o[2]);
+    o[3] = cmul(o[3], w3);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        v[t] = cadd(e[t], o[t]);
+        v[t + 4] = csub(e[t], o[t]);
+    }
+}
+
+// One pass of radix RX over n points whose sub-transforms have length ns:
+// thread index j of n / RX reads points j + m n/RX and writes
+// (j/ns) ns RX + j%ns + m ns.  tw[t] = exp(-2 pi i t / n).
+template <int RX, bool INV>
+__device__ __forceinline__ void fft_radix(float2* v, int j, int ns, int n, const float2* __restrict__ tw)
+{
+    if (ns > 1) {
+        const int k = j & (ns - 1), s = n / (ns * RX);
+#pragma unroll
+        for (int m = 1; m < RX; ++m) {
+            float2 w = __ldg(tw + k * m * s);
+            if (INV) w.y = -w.y;
+            v[m] = cmul(v[m], w);
+        }
+    }
+    if (RX == 8) fft8<INV>(v);
+    else if (RX == 4) fft4<INV>(v);
+    else fft2<INV>(v[0], v[1]);
+}
+
+// The passes of one direction over the thread's 8 points.  get(i) yields
+// point i of the first pass, put(i, v) takes point i of the last; in between
+// the points go through sh.  The sub-transform lengths are 1, 8, 64, ...; a
+// last pass of radix 2 or 4 does 4 or 2 of them per thread.
+template <bool INV, typename G, typename P>
+__device__ __forceinline__ void fft_passes(float2* sh, int n, int log2n, const float2* __restrict__ tw, G get, P put)
+{
+    const int j = threadIdx.x, T = n >> 3;
+    float2 v[8];
+    int ns = 1;
+    for (int left = log2n; left > 0;) {
+        const bool first = ns == 1;
+        const int lr = left >= 3 ? 3 : left;
+        const bool last = left == lr;
+        if (!first) __syncthreads();   // the previous pass's stores
+        if (lr == 3) {
+#pragma unroll
+            for (int m = 0; m < 8; ++m) v[m] = first ? get(j + m * T) : sh[fft_pad(j + m * T)];
+            fft_radix<8, INV>(v, j, ns, n, tw);
+            if (!first) __syncthreads();   // every load done
+            const int base = (j / ns) * ns * 8 + (j & (ns - 1));
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                if (last) put(base + m * ns, v[m]);
+                else sh[fft_pad(base + m * ns)] = v[m];
+            }
+        } else if (lr == 2) {   // two radix-4 butterflies: j and j + T
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) v[4 * h + m] = sh[fft_pad(j + h * T + m * 2 * T)];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int jj = j + h * T;
+                fft_radix<4, INV>(v + 4 * h, jj, ns, n, tw);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) put((jj / ns) * ns * 4 + (jj & (ns - 1)) + m * ns, v[4 * h + m]);
+            }
+        } else {
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+#pragma unroll
+                for (int m = 0; m < 2; ++m) v[2 * h + m] = sh[fft_pad(j + h * T + m * 4 * T)];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const int jj = j + h * T;
+                fft_radix<2, INV>(v + 2 * h, jj, ns, n, tw);
+#pragma unroll
+                for (int m = 0; m < 2; ++m) put((jj / ns) * ns * 2 + (jj & (ns - 1)) + m * ns, v[2 * h + m]);
+            }
+        }
+        ns <<= lr;
+        left -= lr;
+    }
+}
+
+// rows 2 blockIdx.x and 2 blockIdx.x + 1 of nrows rows of R values (row % ZP is
+// the detector row): out = ramp(weight * in).  n / 8 threads.  H[k] / n is the
+// taps' spectrum in sp.
+__global__ void __launch_bounds__(kFftMost / 8)
+k_ramp_fft(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ weight,
+           const float2* __restrict__ tw, const float* __restrict__ sp, int R, int ZP, long long nrows, int n, int log2n)
+{
+    extern __shared__ float2 fsh[];
+    const long long r0 = 2LL * blockIdx.x;
+    const bool two = r0 + 1 < nrows;
+    const float* __restrict__ a = in + r0 * R;
+    const float* __restrict__ wa = weight + (r0 % ZP) * R;
+    const float* __restrict__ wb = weight + ((r0 + 1) % ZP) * R;
+    auto read = [&](int i) {
+        if (i >= R) return make_float2(0.0f, 0.0f);
+        return make_float2(__ldg(a + i) * __ldg(wa + i), two ? __ldg(a + R + i) * __ldg(wb + i) : 0.0f);
+    };
+    // the spectrum goes back through shared memory in order
+    fft_passes<false>(fsh, n, log2n, tw, read, [&](int i, float2 v) {
+        const float h = __ldg(sp + i);
+        fsh[n + (n >> 3) + fft_pad(i)] = make_float2(v.x * h, v.y * h);
+    });
+    __syncthreads();
+    float* __restrict__ o = out + r0 * R;
+    fft_passes<true>(fsh, n, log2n, tw, [&](int i) { return fsh[n + (n >> 3) + fft_pad(i)]; }, [&](int i, float2 v) {
+        if (i < R) {
+            o[i] = v.x;
+            if (two) o[R + i] = v.y;
+        }
+    });
+}
+
+static constexpr int FB_BX = 32, FB_BY = 4, FB_K = 8;
 
 // floor(x) and (int)floor(x) for 0 <= x < 2^22 without conversion
 // instructions (the backprojection is bound by the pipe that executes them):
@@ -112,8 +280,26 @@ __device__ __forceinline__ float floor_small(float x, int& n)
     }
     return r;
 }
+// x / d, correctly rounded, from r = 1/d correctly rounded: one multiplication
+// and two fused multiply-adds (Markstein's division; Brisebarre, Muller and
+// Raina, IEEE Trans. Computers 53(8), 2004, for a divisor known in advance).
+// The remainder must not underflow; the launcher checks the geometry's scale
+// (RCP) and the divisions are written out otherwise.  Compared with x / d on
+// 1.2e9 pairs of random mantissas: no difference.
+template <bool RCP> __device__ __forceinline__ float div_by(float x, float d, float r)
+{
+    if (!RCP) return fdv(x, d);
+    const float q = fm(x, r);
+    return __fmaf_rn(__fmaf_rn(-d, q, x), r, q);
+}
+
+// FULL: a full circle (us_rate*Nviews == 360).  Three divisions per voxel and
+// view (by the voxel column's distance, DSO and the row pitch) by div_by, what
+// does not depend on z once per FB_K voxels.  Bound by issue; 32 views into
+// 512^3: 7.3 ms (13.6 ms with IEEE divide sequences and 4 voxels a thread).
+template <bool FULL, bool RCP>
 __global__ void __launch_bounds__(FB_BX * FB_BY)
-k_fdk_bp(const DevGeom g, float* __restrict__ vol, const float* __restrict__ proj, int view0, int nview)
+k_fdk_bp(const __grid_constant__ DevGeom g, float* __restrict__ vol, const float* __restrict__ proj, int view0, int nview)
 {
     const int i = blockIdx.x * FB_BX + (threadIdx.x % FB_BX);
     const int j = blockIdx.y * FB_BY + (threadIdx.x / FB_BX);
@@ -121,50 +307,51 @@ k_fdk_bp(const DevGeom g, float* __restrict__ vol, const float* __restrict__ pro
     if (i >= g.M || j >= g.N) return;
     const long long MN = (long long)g.M * g.N;
     const int R = g.R, ZP = g.ZP;
-    const float DSO = g.dso, DOD = g.dod;
+    const float DSO = g.dso, SDD = fs(g.dso, g.dod), Rf = (float)R, ZPf = (float)ZP;
+    const float r_dso = __frcp_rn(DSO), r_du = __frcp_rn(g.du), r_dv = __frcp_rn(g.dv);
     // kernel_FDK.cu:86-88
     const float x = fa(fa(g.bx, fm(g.vx, 0.5f)), fm((float)i, g.vx));
     const float y = fa(fa(g.by, fm(g.vy, 0.5f)), fm((float)j, g.vy));
-    float acc[FB_K], zc[FB_K];
+    float acc[FB_K], dz[FB_K];
 #pragma unroll
     for (int kk = 0; kk < FB_K; ++kk) {
         const int k = min(k0 + kk, g.Z - 1);
         acc[kk] = vol[(long long)k * MN + (long long)j * g.M + i];
-        zc[kk] = fa(fa(g.bz, fm(g.vz, 0.5f)), fm((float)k, g.vz));
+        dz[kk] = fm(DSO, fa(fa(g.bz, fm(g.vz, 0.5f)), fm((float)k, g.vz)));
     }
     for (int w = 0; w < nview; ++w) {
         const float2 scv = g.trig_fdk[view0 + w];
         const float sn = scv.x, cs = scv.y;
         const float t = fa(fm(x, cs), fm(y, sn));
         const float s = fa(fm(-x, sn), fm(y, cs));
-        const float ds = fs(DSO, s);
+        const float ds = fs(DSO, s), r_ds = __frcp_rn(ds);
         const float temp1 = fdv(fm(DSO, DSO), fm(ds, ds));
-        float p = fdv(fm(DSO, t), ds);
-        p = fdv(fs(fdv(fm(p, fs(DSO, DOD)), DSO), g.ymin), g.du);
-        const float* __restrict__ pv = proj + (long long)w * R * ZP;
+        float p = div_by<RCP>(fm(DSO, t), ds, r_ds);
+        p = div_by<RCP>(fs(div_by<RCP>(fm(p, SDD), DSO, r_dso), g.ymin), g.du, r_du);
+        const bool in_u = (0 <= p) && (fa(p, 1.0f) < Rf);
+        int bn;
+        const float bn0 = fs(p, floor_small(in_u ? p : 0.0f, bn)), bn1 = fs(1.0f, bn0);
+        const float* __restrict__ pv = proj + (long long)w * R * ZP + bn;
 #pragma unroll
         for (int kk = 0; kk < FB_K; ++kk) {
-            float ksi = fdv(fm(DSO, zc[kk]), ds);
-            ksi = fdv(fs(fdv(fm(ksi, fs(DSO, DOD)), DSO), g.zmin), g.dv);
-            float temp2;
-            if ((0 <= ksi) && (fa(ksi, 1.0f) < (float)ZP) && (0 <= p) && (fa(p, 1.0f) < (float)R)) {
-                int an, bn;
-                const float an0 = fs(ksi, floor_small(ksi, an));   // ksi - an, an = floor(ksi)
-                const float bn0 = fs(p, floor_small(p, bn));
-                const float* q0 = pv + (long long)R * an + bn;
+            float ksi = div_by<RCP>(dz[kk], ds, r_ds);
+            ksi = div_by<RCP>(fs(div_by<RCP>(fm(ksi, SDD), DSO, r_dso), g.zmin), g.dv, r_dv);
+            float temp2 = 0.0f;
+            if ((0 <= ksi) && (fa(ksi, 1.0f) < ZPf) && in_u) {
+                int an;
+                const float an0 = fs(ksi, floor_small(ksi, an)), an1 = fs(1.0f, an0);   // ksi - an, an = floor(ksi)
+                const float* q0 = pv + R * an;
                 const float* q1 = q0 + R;
-                const float t00 = fm(fm(fs(1.0f, an0), fs(1.0f, bn0)), __ldg(q0));
-                const float t01 = fm(fm(fs(1.0f, an0), bn0), __ldg(q0 + 1));
-                const float t10 = fm(fm(an0, fs(1.0f, bn0)), __ldg(q1));
+                const float t00 = fm(fm(an1, bn1), __ldg(q0));
+                const float t01 = fm(fm(an1, bn0), __ldg(q0 + 1));
+                const float t10 = fm(fm(an0, bn1), __ldg(q1));
                 const float t11 = fm(fm(an0, bn0), __ldg(q1 + 1));
                 temp2 = fa(fa(fa(t00, t01), t10), t11);
-            } else {
-                temp2 = 0.0f;
             }
             // vol += temp1*temp2*(us_rate*PI/180.0f)*360.0/(us_rate*Nviews)  (float*float*float, then double)
             const float fprod = fm(fm(temp1, temp2), g.fdk_ang);
-            if (g.fdk_full) {
-                // a full circle (us_rate*Nviews == 360): (double)fprod*360.0 is exact
+            if (FULL) {
+                // a full circle: (double)fprod*360.0 is exact
                 // (24 + 6 significant bits) and dividing it by 360 gives fprod back; and
                 // the FP64 sum of two floats rounded to float is their float sum (when
                 // the FP64 sum is inexact the smaller term is below 2^-28 of the larger,
@@ -198,15 +385,51 @@ static void ramp_taps(const ctr_geometry_desc& d, std::vector<float>& taps)
         H[i] = hv;
     }
     taps.assign(2 * R - 1, 0.f);
-    for (int n = -(R - 1); n <= R - 1; ++n) {
+    std::vector<double> cosine(P);
+    for (int m = 0; m < P; ++m) cosine[m] = std::cos(2.0 * M_PI * (double)m / (double)P);
+    for (int n = 0; n <= R - 1; ++n) {
         double acc = 0.0;
-        const long long an = n < 0 ? -n : n;
-        for (int i = 0; i < P; ++i) {
-            const long long m = ((long long)i * an) % P;
-            acc += (double)H[i] * std::cos(2.0 * M_PI * (double)m / (double)P);
-        }
-        taps[n + R - 1] = (float)(acc / (double)P);
+        for (int i = 0, m = 0; i < P; ++i, m = m + n < P ? m + n : m + n - P) acc += (double)H[i] * cosine[m];   // m = i n mod P
+        taps[R - 1 + n] = taps[R - 1 - n] = (float)(acc / (double)P);
     }
+}
+
+// Tables of k_ramp_fft, one allocation: n twiddles exp(-2 pi i t / n), the taps'
+// spectrum / n, the cosine weights [v][u] (kernel_FDK.cu:1-14).
+static size_t fft_points(int R)
+{
+    size_t n = 8;
+    while (n < 2 * (size_t)R - 1) n <<= 1;
+    return n;
+}
+static ctr_status fft_tables(Geometry& G, const std::vector<float>& taps)
+{
+    const int R = G.desc.nu, ZP = G.dg.ZP;
+    const size_t n = fft_points(R);
+    std::vector<float> h(3 * n + (size_t)R * ZP);
+    std::vector<double> cosine(n);
+    for (size_t t = 0; t < n; ++t) {
+        const double a = 2.0 * M_PI * (double)t / (double)n;
+        cosine[t] = std::cos(a);
+        h[2 * t] = (float)cosine[t];
+        h[2 * t + 1] = (float)-std::sin(a);
+    }
+    for (size_t k = 0; k <= n / 2; ++k) {
+        double acc = taps[R - 1];
+        for (int m = 1; m < R; ++m) acc += 2.0 * (double)taps[R - 1 + m] * cosine[(k * (size_t)m) & (n - 1)];
+        h[2 * n + k] = h[2 * n + ((n - k) & (n - 1))] = (float)(acc / (double)n);
+    }
+    const DevGeom& g = G.dg;
+    const double mag = (double)g.dso / ((double)g.dso - (double)g.dod);
+    for (int v = 0; v < ZP; ++v)
+        for (int u = 0; u < R; ++u) {
+            const double x2 = ((double)g.ymin + (double)u * g.du) * mag, x3 = ((double)g.zmin + (double)v * g.dv) * mag;
+            h[3 * n + (size_t)v * R + u] =
+                (float)((double)g.dso / std::sqrt((double)g.dso * g.dso + x2 * x2 + x3 * x3));
+        }
+    CTR_CUDA_TRY(cudaMalloc(&G.d_ramp, h.size() * sizeof(float)));
+    CTR_CUDA_TRY(cudaMemcpy(G.d_ramp, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
+    return CTR_OK;
 }
 
 ctr_status launch_fdk(Geometry& G, const float* sino, float* vol, cudaStream_t st)
@@ -214,13 +437,19 @@ ctr_status launch_fdk(Geometry& G, const float* sino, float* vol, cudaStream_t s
     const DevGeom& g = G.dg;
     const int nv = g.nviews;
     const long long P = G.npix();
+    const size_t n = fft_points(g.R);
+    const bool fft = n <= (size_t)kFftMost;
     if (!G.d_ramp) {
         std::vector<float> taps;
         ramp_taps(G.desc, taps);
-        CTR_CUDA_TRY(cudaMalloc(&G.d_ramp, taps.size() * sizeof(float)));
-        CTR_CUDA_TRY(cudaMemcpy(G.d_ramp, taps.data(), taps.size() * sizeof(float), cudaMemcpyHostToDevice));
+        if (fft) {
+            CTR_TRY(fft_tables(G, taps));
+        } else {
+            CTR_CUDA_TRY(cudaMalloc(&G.d_ramp, taps.size() * sizeof(float)));
+            CTR_CUDA_TRY(cudaMemcpy(G.d_ramp, taps.data(), taps.size() * sizeof(float), cudaMemcpyHostToDevice));
+        }
     }
-    const size_t need = (size_t)P * nv * 2;
+    const size_t need = (size_t)P * nv * (fft ? 1 : 2);
     if (G.fdk_cap < need) {
         if (G.d_fdk) cudaFree(G.d_fdk);
         G.d_fdk = nullptr;
@@ -228,17 +457,29 @@ ctr_status launch_fdk(Geometry& G, const float* sino, float* vol, cudaStream_t s
         CTR_CUDA_TRY(cudaMalloc(&G.d_fdk, need * sizeof(float)));
         G.fdk_cap = need;
     }
-    float* wsino = G.d_fdk;
-    float* fsino = G.d_fdk + (size_t)P * nv;
-    for (int v0 = 0; v0 < nv; v0 += 65535) {
-        const int cnt = std::min(65535, nv - v0);
-        k_fdk_weight<<<dim3((g.R + 127) / 128, g.ZP, cnt), 128, 0, st>>>(g, sino + (size_t)P * v0, wsino + (size_t)P * v0);
-    }
+    float* fsino = G.d_fdk;
     const long long nrows = (long long)nv * g.ZP;
-    for (long long r0 = 0; r0 < nrows; r0 += 65535LL * RP_ROWS) {
-        const long long cnt = std::min<long long>(65535LL * RP_ROWS, nrows - r0);
-        dim3 grd((g.R + RP_COLS - 1) / RP_COLS, (unsigned)((cnt + RP_ROWS - 1) / RP_ROWS));
-        k_ramp<<<grd, 128, 0, st>>>(wsino + r0 * g.R, fsino + r0 * g.R, G.d_ramp, g.R, cnt);
+    if (fft) {
+        int log2n = 0;
+        while ((1u << log2n) < n) ++log2n;
+        const size_t smem = 2 * (n + (n >> 3)) * sizeof(float2);
+        CTR_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(&k_ramp_fft),
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        const float2* tw = (const float2*)G.d_ramp;
+        const float* sp = G.d_ramp + 2 * n;
+        k_ramp_fft<<<(unsigned)((nrows + 1) / 2), (unsigned)(n / 8), smem, st>>>(sino, fsino, sp + n, tw, sp, g.R, g.ZP,
+                                                                                nrows, (int)n, log2n);
+    } else {
+        float* wsino = G.d_fdk + (size_t)P * nv;
+        for (int v0 = 0; v0 < nv; v0 += 65535) {
+            const int cnt = std::min(65535, nv - v0);
+            k_fdk_weight<<<dim3((g.R + 127) / 128, g.ZP, cnt), 128, 0, st>>>(g, sino + (size_t)P * v0, wsino + (size_t)P * v0);
+        }
+        for (long long r0 = 0; r0 < nrows; r0 += 65535LL * RP_ROWS) {
+            const long long cnt = std::min<long long>(65535LL * RP_ROWS, nrows - r0);
+            dim3 grd((g.R + RP_COLS - 1) / RP_COLS, (unsigned)((cnt + RP_ROWS - 1) / RP_ROWS));
+            k_ramp<<<grd, 128, 0, st>>>(wsino + r0 * g.R, fsino + r0 * g.R, G.d_ramp, g.R, cnt);
+        }
     }
     CTR_CUDA_TRY(cudaGetLastError());
     return launch_fdk_bp(G, fsino, 0, nv, vol, st);
@@ -268,9 +509,22 @@ ctr_status launch_fdk_bp(const Geometry& G, const float* fsino, int view0, int n
     const DevGeom& g = G.dg;
     const long long P = G.npix();
     dim3 grd((g.M + FB_BX - 1) / FB_BX, (g.N + FB_BY - 1) / FB_BY, (g.Z + FB_K - 1) / FB_K);
+    // div_by: lengths far from the ends of the float range
+    auto plain = [](float v) { return std::fabs(v) > 1e-9f && std::fabs(v) < 1e9f; };
+    const bool rcp = plain(g.dso) && plain(g.dsod) && plain(g.du) && plain(g.dv) && plain(g.vx) && plain(g.vy) && plain(g.vz);
     const int VB = 32;
-    for (int w = 0; w < nview; w += VB)
-        k_fdk_bp<<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, fsino + (size_t)P * w, view0 + w, std::min(VB, nview - w));
+    for (int w = 0; w < nview; w += VB) {
+        const float* f = fsino + (size_t)P * w;
+        const int n = std::min(VB, nview - w);
+        if (!rcp) {
+            if (g.fdk_full) k_fdk_bp<true, false><<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, f, view0 + w, n);
+            else k_fdk_bp<false, false><<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, f, view0 + w, n);
+        } else if (g.fdk_full) {
+            k_fdk_bp<true, true><<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, f, view0 + w, n);
+        } else {
+            k_fdk_bp<false, true><<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, f, view0 + w, n);
+        }
+    }
     CTR_CUDA_TRY(cudaGetLastError());
     return CTR_OK;
 }
