@@ -3,11 +3,14 @@
 // FGP restates FGP_denoise_GPUx7_exact (V63/host_FGP_Denoise_GPUx7.c:1-111)
 // and its kernels FGP_operator_L_Pc / FGP_operator_LT_Pp
 // (V63/kernel_FGP_Denoise_GPUx7.cu:2-88) with the same float operations.  The
-// duals are stored in the volume's storage type; L stays FP32.
+// duals are stored in the volume's storage type; L is FP32 and never stored.
 //
 // Dual layout: volume-sized arrays; r[p] belongs to the edge (x, x+1) and is 0
 // at x = nx-1 (the reference's zero-padded d_r[x+1], V63/host_FGP_Denoise_
 // GPUx7.c:8-38); likewise s along y and t along z.
+#include <algorithm>
+#include <type_traits>
+
 #include "ctr_device.cuh"
 
 namespace ctr {
@@ -28,79 +31,177 @@ __device__ __forceinline__ float fgp_L(const TF* __restrict__ f, const T* __rest
     return fs(Store<TF>::ld(f + p), fm(lambda, tl));                   // :17
 }
 
-// One inner iteration in two passes, as the reference's x7 form: k_fgp_L
-// writes L = f - lambda*div(r,s,t) (FP32, as the reference keeps it) for every
-// voxel; k_fgp_dual reads L at the voxel and its +x, +y, +z neighbours and
-// updates the voxel's own duals in place (no voxel reads another's duals in
-// this pass, so no double buffer is needed).  One thread per voxel, a 3-D
-// grid of 32x8 tiles: both passes stream at close to the copy bandwidth.
-template <typename T, typename TF = T>
-__global__ void __launch_bounds__(FG_BX * FG_BY)
-k_fgp_L(int M, int N, int Z, const TF* __restrict__ f, const T* __restrict__ r, const T* __restrict__ s,
-        const T* __restrict__ t, float* __restrict__ L, float lambda)
+// x / d correctly rounded from r = 1/d correctly rounded (Markstein's division;
+// Brisebarre, Muller and Raina, IEEE Trans. Computers 53(8), 2004), where the
+// remainder cannot underflow and the quotient is finite; the plain division
+// elsewhere.  1 <= d.
+__device__ __forceinline__ float div_exact(float x, float d, float r)
 {
-    const int x = blockIdx.x * FG_BX + threadIdx.x;
-    const int y = blockIdx.y * FG_BY + threadIdx.y;
-    const int z = blockIdx.z;
-    if (x >= M || y >= N) return;
-    const long long MN = (long long)M * N;
-    const long long p = (long long)z * MN + (long long)y * M + x;
-    L[p] = fgp_L<T, TF>(f, r, s, t, x, y, z, p, M, MN, lambda);          // L_Pc, GPUx7.cu:2-24
+    const float q = fm(x, r);
+    const float y = __fmaf_rn(__fmaf_rn(-d, q, x), r, q);
+    const float m = fabsf(x);
+    return (m > 1e-30f && m < 1e30f && d < 1e30f) ? y : fdv(x, d);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(FG_BX * FG_BY)
-k_fgp_dual(int M, int N, int Z, const float* __restrict__ L, T* __restrict__ r, T* __restrict__ s,
-           T* __restrict__ t, T* __restrict__ o, T* __restrict__ pd, T* __restrict__ q, float alpha12, float gam)
+// One inner iteration in one pass: L = f - lambda*div(r,s,t) (L_Pc,
+// V63/kernel_FGP_Denoise_GPUx7.cu:2-24) and the dual step from L at the voxel
+// and its +x, +y, +z neighbours (LT_Pp, :52-86).  A block marches a 32x8 tile
+// through a run of z planes; L of the next plane goes to shared memory (never
+// to HBM), L of this plane and the duals read for it stay in registers.  Warp
+// 8 computes the tile's two edges (the row below and the column to the right)
+// while the others update their voxels.  What the next plane reads is loaded
+// before the barrier of this one.  Neighbours' duals are read, so the
+// new ones go to another set of arrays.
+//
+// Bound by HBM bandwidth and latency in FP32 (4.3 TB/s of 6.5), by issue and
+// latency with 16-bit duals (66 % of the issue slots).  FP32 duals: the extrapolated r_k = o_k + g (o_k - o_(k-1)) is
+// formed from the two stored projections with the operations that stored it,
+// so r, s, t are never written: f and six arrays in, three out, 40 bytes a
+// voxel.  16-bit duals keep r, s, t as stored (their rounding differs from
+// one formed from the rounded o): 26 bytes a voxel.  The two-pass form (L
+// through HBM) moved 72 and 40 bytes.  An iteration: 512^3 FP32 1.25 ms
+// (2.15 ms in two passes), 333x257x190 BF16 0.176 ms (0.245 ms).
+template <typename T> struct FgpSet {
+    static constexpr bool REC = std::is_same<T, float>::value;
+    const T* r[3];    // REC: o_k, p_k, q_k;         else r, s, t
+    const T* r0[3];   // REC: o_(k-1), ...;          else unused
+    T* rn[3];         // REC: o_(k+1), ...;          else the next r, s, t
+    T* o[3];          // else: o, p, q, updated in place
+};
+
+template <typename T, typename TF, bool FIRST>
+__global__ void __launch_bounds__(32 * (FG_BY + 1), 4)
+k_fgp_step(int M, int N, int Z, int zrun, const TF* __restrict__ f, const FgpSet<T> d, float lambda, float alpha12,
+           float gam, float gam_prev)
 {
-    const int x = blockIdx.x * FG_BX + threadIdx.x;
-    const int y = blockIdx.y * FG_BY + threadIdx.y;
-    const int z = blockIdx.z;
-    if (x >= M || y >= N) return;
-    const long long MN = (long long)M * N;
-    const long long p = (long long)z * MN + (long long)y * M + x;
-    const float Lc = __ldg(L + p);
-    const float Lx = (x < M - 1) ? __ldg(L + p + 1) : 0.0f;
-    const float Ly = (y < N - 1) ? __ldg(L + p + M) : 0.0f;
-    const float Lz = (z < Z - 1) ? __ldg(L + p + MN) : 0.0f;
-    // LT_Pp (V63/kernel_FGP_Denoise_GPUx7.cu:52-86)
-    float tr = Store<T>::ldw(r + p), ts = Store<T>::ldw(s + p), tt = Store<T>::ldw(t + p);
-    if (x < M - 1) tr = fa(tr, fm(alpha12, fs(Lc, Lx)));
-    if (y < N - 1) ts = fa(ts, fm(alpha12, fs(Lc, Ly)));
-    if (z < Z - 1) tt = fa(tt, fm(alpha12, fs(Lc, Lz)));
-    const float rst = __fsqrt_rn(fa(fa(fm(tr, tr), fm(ts, ts)), fm(tt, tt)));
-    const float den = fmaxf(1.0f, rst);
-    if (x < M - 1) {
-        const float on = fdv(tr, den);
-        Store<T>::st(r + p, fa(on, fm(gam, fs(on, Store<T>::ldw(o + p)))));
-        Store<T>::st(o + p, on);
+    constexpr bool REC = FgpSet<T>::REC;
+    __shared__ float sL[2][FG_BY + 1][33];   // [plane parity][row][column]
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int x0 = blockIdx.x * FG_BX, y0 = blockIdx.y * FG_BY;
+    const int zb = blockIdx.z * zrun, ze = min(Z, zb + zrun);
+    const unsigned MN = (unsigned)M * (unsigned)N;   // voxel indices are below 2^31
+    // what L at a voxel reads, loaded a plane ahead: f, the voxel's duals, r at
+    // x-1 and s at y-1 (REC: o_k in a, o_(k-1) in b)
+    struct Raw { float f, a[5], b[5]; };
+    auto load = [&](Raw& w, bool on, int x, int y, unsigned p) {
+        const unsigned q[5] = {p, p, p, p - 1u, p - (unsigned)M};
+        const bool has[5] = {on, on, on, on && x > 0, on && y > 0};
+        w.f = on ? Store<TF>::ld(f + p) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const int a = i < 3 ? i : i - 3;
+            w.a[i] = w.b[i] = 0.0f;
+            if (!FIRST && has[i]) {
+                w.a[i] = Store<T>::ld(d.r[a] + q[i]);
+                if (REC) w.b[i] = Store<T>::ld(d.r0[a] + q[i]);
+            }
+        }
+    };
+    // the dual a step reads: as stored, or extrapolated from o_k and o_(k-1)
+    auto extrap = [&](float o1, float o0) { return REC ? fa(o1, fm(gam_prev, fs(o1, o0))) : o1; };
+    // L (L_Pc :14-17); the voxel's duals to rst, t of the plane below in tm
+    auto L_of = [&](const Raw& w, float tm, float rst[3]) -> float {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) rst[i] = extrap(w.a[i], w.b[i]);
+        const float tl = fa(fa(fs(rst[0], extrap(w.a[3], w.b[3])), fs(rst[1], extrap(w.a[4], w.b[4]))), fs(rst[2], tm));
+        return fs(w.f, fm(lambda, tl));
+    };
+    auto t_below = [&](bool on, unsigned p) -> float {   // t at (x, y, zb - 1)
+        if (FIRST || !on || zb == 0) return 0.0f;
+        return extrap(Store<T>::ld(d.r[2] + p - MN), REC ? Store<T>::ld(d.r0[2] + p - MN) : 0.0f);
+    };
+    if (ty == FG_BY) {   // the edges: row y0+8 (32 columns), then column x0+32 (8 rows)
+        const int xe = x0 + tx, ye = y0 + FG_BY, xc = x0 + FG_BX, yc = y0 + tx;
+        const bool row = xe < M && ye < N, colm = tx < FG_BY && xc < M && yc < N;
+        unsigned pr = (unsigned)zb * MN + (unsigned)ye * M + xe, pc = (unsigned)zb * MN + (unsigned)yc * M + xc;
+        float tr = t_below(row, pr), tc = t_below(colm, pc), u[3];
+        Raw wr, wc;
+        load(wr, row, xe, ye, pr);
+        load(wc, colm, xc, yc, pc);
+        for (int z = zb; z < ze; ++z) {
+            const float Lr = L_of(wr, tr, u);
+            tr = u[2];
+            const float Lk = L_of(wc, tc, u);
+            tc = u[2];
+            pr += MN;
+            pc += MN;
+            load(wr, row && z + 1 < ze, xe, ye, pr);
+            load(wc, colm && z + 1 < ze, xc, yc, pc);
+            if (row) sL[z & 1][FG_BY][tx] = Lr;
+            if (colm) sL[z & 1][tx][32] = Lk;
+            __syncthreads();
+        }
+        return;
     }
-    if (y < N - 1) {
-        const float pn = fdv(ts, den);
-        Store<T>::st(s + p, fa(pn, fm(gam, fs(pn, Store<T>::ldw(pd + p)))));
-        Store<T>::st(pd + p, pn);
-    }
-    if (z < Z - 1) {
-        const float qn = fdv(tt, den);
-        Store<T>::st(t + p, fa(qn, fm(gam, fs(qn, Store<T>::ldw(q + p)))));
-        Store<T>::st(q + p, qn);
+    const int x = x0 + tx, y = y0 + ty;
+    const bool in = x < M && y < N;
+    const bool ex = x < M - 1, ey = y < N - 1;
+    unsigned p = (unsigned)zb * MN + (unsigned)y * M + x;
+    float cur[3], nxt[3] = {0.f, 0.f, 0.f}, Ln = 0.0f;
+    Raw w;
+    load(w, in, x, y, p);
+    float Lc = L_of(w, t_below(in, p), cur);
+    load(w, in && zb + 1 < Z, x, y, p + MN);
+    float ahead[3] = {0.f, 0.f, 0.f};   // not REC: o, p, q of the plane to come
+    auto load_o = [&](bool on, unsigned q) {
+        if (!REC && !FIRST && on)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) ahead[a] = Store<T>::ldw(d.o[a] + q);
+    };
+    load_o(in, p);
+    for (int z = zb; z < ze; ++z, p += MN) {
+        sL[z & 1][ty][tx] = Lc;
+        const bool ez = z < Z - 1;
+        const float old[3] = {ahead[0], ahead[1], ahead[2]};
+        load_o(in && z + 1 < ze, p + MN);
+        Ln = L_of(w, cur[2], nxt);
+        load(w, in && z + 1 < ze && z + 2 < Z, x, y, p + 2u * MN);   // (the run's last plane needs L one plane up)
+        __syncthreads();   // the other parity's plane is not written before the next barrier
+        if (in) {
+            float tr = cur[0], ts = cur[1], tt = cur[2];
+            if (ex) tr = fa(tr, fm(alpha12, fs(Lc, sL[z & 1][ty][tx + 1])));
+            if (ey) ts = fa(ts, fm(alpha12, fs(Lc, sL[z & 1][ty + 1][tx])));
+            if (ez) tt = fa(tt, fm(alpha12, fs(Lc, Ln)));
+            // :78-86.  The divisor max(1, sqrt(n)) is 1 unless n > 1; otherwise one
+            // reciprocal serves the three divisions
+            const float n = fa(fa(fm(tr, tr), fm(ts, ts)), fm(tt, tt));
+            float v[3] = {tr, ts, tt};
+            if (n > 1.0f) {
+                const float den = __fsqrt_rn(n), rcp = __frcp_rn(den);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) v[a] = div_exact(v[a], den, rcp);
+            }
+            const bool e[3] = {ex, ey, ez};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float on = e[a] ? v[a] : 0.0f;   // an edge that leaves the volume has no dual
+                if (REC) {
+                    Store<T>::st(d.rn[a] + p, on);
+                } else {
+                    Store<T>::st(d.rn[a] + p, e[a] ? fa(on, fm(gam, fs(on, old[a]))) : 0.0f);
+                    Store<T>::st(d.o[a] + p, on);
+                }
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) cur[a] = nxt[a];
+        Lc = Ln;
     }
 }
 
 // x* = f - lambda*div(o,p,q) (the final L_Pc, V63/host_FGP_Denoise_GPUx7.c:83);
 // with FISTA fused: y = x* + gam*(x* - xprev), xprev = x* (V63/main_recon.cu:375-382).
 template <typename T, bool FISTA>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(FG_BX * FG_BY)
 k_fgp_final(int M, int N, int Z, T* __restrict__ vol, const T* __restrict__ o, const T* __restrict__ pd,
             const T* __restrict__ q, float lambda, T* __restrict__ xprev, float gam, const float* __restrict__ gam_dev)
 {
     if (FISTA && gam_dev) gam = *gam_dev;
+    const int x = blockIdx.x * FG_BX + threadIdx.x, y = blockIdx.y * FG_BY + threadIdx.y;
+    if (x >= M || y >= N) return;
     const long long MN = (long long)M * N;
-    const long long n = MN * Z;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(p % M);
-        const int y = (int)((p / M) % N);
-        const int z = (int)(p / MN);
+    for (int z = blockIdx.z; z < Z; z += gridDim.z) {
+        const long long p = (long long)z * MN + (long long)y * M + x;
         const float xs = fgp_L<T>(vol, o, pd, q, x, y, z, p, M, MN, lambda);
         if (FISTA) {
             const float xp = Store<T>::ldw(xprev + p);
@@ -116,9 +217,6 @@ k_fgp_final(int M, int N, int Z, T* __restrict__ vol, const T* __restrict__ o, c
     }
 }
 
-// Refinement solver: the FP32 input of the prox, y_k + d = (1+g) x_k - g x_(k-1) + d,
-// written over x_(k-1) (which is not needed after it).  d is read in the
-// projectors' tiled layout.
 // Refinement solver: the start d0 of the correction volume, the storage
 // rounding of y_k - y~_k = (1+g)(x_k - x~_k) - g (x_(k-1) - x~_(k-1)), where
 // x~ are the projectors' round-to-nearest copies of the FP32 iterates (the
@@ -159,7 +257,8 @@ k_refine_start(const DevGeom g, const float* __restrict__ xk, const float* __res
     }
 }
 
-// z = y_k + (d - d0) in FP32 into xm (FGP's input).
+// The FP32 input of the prox, z = y_k + (d - d0), written over x_(k-1) (which is
+// not needed after it).  d is read in the projectors' tiled layout.
 template <typename T, typename TD>
 __global__ void __launch_bounds__(256)
 k_refine_sum(const DevGeom g, const float* __restrict__ xk, float* __restrict__ xm, const TD* __restrict__ d,
@@ -220,36 +319,76 @@ static int grid_for(long long n, int threads)
 // t_k = (1 + sqrt(1 + 4 t^2))/2 in float (V63/host_FGP_Denoise_GPUx7.c:161)
 static float next_t(float t) { return (1.0f + sqrtf(1.0f + 4.0f * t * t)) / 2.0f; }
 
+// The inner iterations of the prox of f: duals from zero, the last projections
+// o, p, q in D.  The geometry's workspace holds nine arrays of V duals.
+template <typename T, typename TF>
+static ctr_status fgp_iterations(Geometry& G, const TF* f, float lambda, int iters, T* D[3], cudaStream_t st)
+{
+    const int M = G.desc.nx, N = G.desc.ny, Z = G.desc.nz;
+    const long long V = G.nvox();
+    CTR_TRY(ensure_fgp(&G, fgp_workspace_bytes(V, DT<T>::v)));
+    T* base = (T*)G.d_fgp;
+    T* A[3][3];   // [set][r s t]
+    for (int i = 0; i < 3; ++i)
+        for (int a = 0; a < 3; ++a) A[i][a] = base + (size_t)(3 * i + a) * V;
+    for (int a = 0; a < 3; ++a) D[a] = A[0][a];
+    if (iters <= 0) {
+        CTR_CUDA_TRY(cudaMemsetAsync(base, 0, 3 * (size_t)V * sizeof(T), st));
+        return CTR_OK;
+    }
+    const float alpha12 = 1.0f / (lambda * 12.0f);                 // :166
+    // z planes per block: long runs (each recomputes one plane of L) while the
+    // blocks still fill the GPU about three times (148 SMs x 4 blocks)
+    const long long tiles = (long long)((M + FG_BX - 1) / FG_BX) * ((N + FG_BY - 1) / FG_BY);
+    int zrun = 32;
+    while (zrun > 4 && tiles * ((Z + zrun - 1) / zrun) < 148LL * 24) zrun >>= 1;
+    zrun = std::max(zrun, (Z + 65534) / 65535);
+    const dim3 blk(32, FG_BY + 1), grd((M + FG_BX - 1) / FG_BX, (N + FG_BY - 1) / FG_BY, (Z + zrun - 1) / zrun);
+    float t_k_1 = 1.0f, gam_prev = 0.0f;
+    for (int it = 0; it < iters; ++it) {
+        const float t_k = next_t(t_k_1);
+        const float gam = (t_k_1 - 1.0f) / t_k;
+        FgpSet<T> d{};
+        for (int a = 0; a < 3; ++a) {
+            if (FgpSet<T>::REC) {   // o_k, o_(k-1), o_(k+1) rotate through the three sets
+                d.r[a] = A[it % 3][a];
+                d.r0[a] = it == 1 ? d.r[a] : A[(it + 2) % 3][a];   // g_1 = 0: o_0 = 0 was never written
+                d.rn[a] = A[(it + 1) % 3][a];
+                D[a] = d.rn[a];
+            } else {
+                d.r[a] = A[1 + it % 2][a];
+                d.rn[a] = A[2 - it % 2][a];
+                d.o[a] = A[0][a];
+            }
+        }
+        if (it == 0) k_fgp_step<T, TF, true><<<grd, blk, 0, st>>>(M, N, Z, zrun, f, d, lambda, alpha12, gam, 0.0f);
+        else k_fgp_step<T, TF, false><<<grd, blk, 0, st>>>(M, N, Z, zrun, f, d, lambda, alpha12, gam, gam_prev);
+        t_k_1 = t_k;
+        gam_prev = gam;
+    }
+    CTR_CUDA_TRY(cudaGetLastError());
+    return CTR_OK;
+}
+
+static dim3 fgp_final_grid(int M, int N, int Z)
+{
+    return dim3((M + FG_BX - 1) / FG_BX, (N + FG_BY - 1) / FG_BY, std::min(Z, 65535));
+}
+
 ctr_status launch_fgp(Geometry& G, void* vol, ctr_dtype dt, float lambda, int iters, void* fista_y,
                       void* fista_xprev, float fista_gamma, cudaStream_t st, const float* gamma_dev)
 {
     const int M = G.desc.nx, N = G.desc.ny, Z = G.desc.nz;
-    const long long V = G.nvox();
-    const size_t es = dtype_size(dt);
-    CTR_TRY(ensure_fgp(&G, fgp_workspace_bytes(V, dt)));
-    CTR_CUDA_TRY(cudaMemsetAsync(G.d_fgp, 0, 6 * (size_t)V * es, st));
-    const float alpha12 = 1.0f / (lambda * 12.0f);                 // :166
-    const dim3 blk(FG_BX, FG_BY), grd((M + FG_BX - 1) / FG_BX, (N + FG_BY - 1) / FG_BY, Z);
+    if (fista_y && fista_y != vol) return set_error(CTR_ERR_INVALID_ARGUMENT, "fused FISTA output must alias the volume");
+    const dim3 blk(FG_BX, FG_BY), grd = fgp_final_grid(M, N, Z);
     CTR_DISPATCH_DTYPE(dt, T, {
-        T* base = (T*)G.d_fgp;
-        T* D[6] = {base, base + V, base + 2 * V, base + 3 * V, base + 4 * V, base + 5 * V};   // r s t o p q
-        float* L = (float*)((char*)G.d_fgp + 6 * (size_t)V * es);
-        float t_k_1 = 1.0f;
-        for (int it = 0; it < iters; ++it) {
-            const float t_k = next_t(t_k_1);
-            const float gam = (t_k_1 - 1.0f) / t_k;
-            k_fgp_L<T><<<grd, blk, 0, st>>>(M, N, Z, (const T*)vol, D[0], D[1], D[2], L, lambda);
-            k_fgp_dual<T><<<grd, blk, 0, st>>>(M, N, Z, L, D[0], D[1], D[2], D[3], D[4], D[5], alpha12, gam);
-            t_k_1 = t_k;
-        }
-        if (fista_y) {
-            if (fista_y != vol) return set_error(CTR_ERR_INVALID_ARGUMENT, "fused FISTA output must alias the volume");
-            k_fgp_final<T, true><<<grid_for(V, 256), 256, 0, st>>>(M, N, Z, (T*)vol, D[3], D[4], D[5], lambda,
-                                                                    (T*)fista_xprev, fista_gamma, gamma_dev);
-        } else {
-            k_fgp_final<T, false><<<grid_for(V, 256), 256, 0, st>>>(M, N, Z, (T*)vol, D[3], D[4], D[5], lambda,
-                                                                     nullptr, 0.0f, nullptr);
-        }
+        T* D[3];
+        CTR_TRY((fgp_iterations<T, T>(G, (const T*)vol, lambda, iters, D, st)));
+        if (fista_y)
+            k_fgp_final<T, true><<<grd, blk, 0, st>>>(M, N, Z, (T*)vol, D[0], D[1], D[2], lambda, (T*)fista_xprev,
+                                                      fista_gamma, gamma_dev);
+        else
+            k_fgp_final<T, false><<<grd, blk, 0, st>>>(M, N, Z, (T*)vol, D[0], D[1], D[2], lambda, nullptr, 0.0f, nullptr);
     });
     CTR_CUDA_TRY(cudaGetLastError());
     return CTR_OK;
@@ -269,9 +408,7 @@ ctr_status launch_momentum(const Geometry& G, void* y, void* xprev, const void* 
 ctr_status launch_refine_update(Geometry& G, float* xk, float* xm, const void* d_tiled, ctr_dtype ddt, void* xt_tiled,
                                 ctr_dtype dt, float lam, int iters, const float* gdev, cudaStream_t st)
 {
-    const int M = G.desc.nx, N = G.desc.ny, Z = G.desc.nz;
     const long long V = G.nvox();
-    const size_t es = dtype_size(dt);
     const bool fgp = lam > 0.f && iters >= 0;
     if (ddt != dt && ddt != CTR_F32) return set_error(CTR_ERR_INVALID_ARGUMENT, "correction type");
     if (fgp) CTR_TRY(ensure_fgp(&G, fgp_workspace_bytes(V, dt)));
@@ -279,25 +416,10 @@ ctr_status launch_refine_update(Geometry& G, float* xk, float* xm, const void* d
     CTR_DISPATCH_DTYPE(dt, T, {
         if (ddt == CTR_F32) k_refine_sum<T, float><<<nb, 256, 0, st>>>(G.dg, xk, xm, (const float*)d_tiled, gdev);
         else k_refine_sum<T, T><<<nb, 256, 0, st>>>(G.dg, xk, xm, (const T*)d_tiled, gdev);
-        if (fgp) {
-            CTR_CUDA_TRY(cudaMemsetAsync(G.d_fgp, 0, 6 * (size_t)V * es, st));
-            const float alpha12 = 1.0f / (lam * 12.0f);
-            const dim3 blk(FG_BX, FG_BY), grd((M + FG_BX - 1) / FG_BX, (N + FG_BY - 1) / FG_BY, Z);
-            T* base = (T*)G.d_fgp;
-            T* D[6] = {base, base + V, base + 2 * V, base + 3 * V, base + 4 * V, base + 5 * V};   // r s t o p q
-            float* L = (float*)((char*)G.d_fgp + 6 * (size_t)V * es);
-            float t_k_1 = 1.0f;
-            for (int it = 0; it < iters; ++it) {
-                const float t_k = next_t(t_k_1);
-                const float gam = (t_k_1 - 1.0f) / t_k;
-                k_fgp_L<T, float><<<grd, blk, 0, st>>>(M, N, Z, xm, D[0], D[1], D[2], L, lam);
-                k_fgp_dual<T><<<grd, blk, 0, st>>>(M, N, Z, L, D[0], D[1], D[2], D[3], D[4], D[5], alpha12, gam);
-                t_k_1 = t_k;
-            }
-            k_refine_final<T, true><<<nb, 256, 0, st>>>(G.dg, xk, xm, D[3], D[4], D[5], lam, (T*)xt_tiled);
-        } else {
-            k_refine_final<T, false><<<nb, 256, 0, st>>>(G.dg, xk, xm, nullptr, nullptr, nullptr, 0.f, (T*)xt_tiled);
-        }
+        T* D[3] = {nullptr, nullptr, nullptr};
+        if (fgp) CTR_TRY((fgp_iterations<T, float>(G, xm, lam, iters, D, st)));
+        if (fgp) k_refine_final<T, true><<<nb, 256, 0, st>>>(G.dg, xk, xm, D[0], D[1], D[2], lam, (T*)xt_tiled);
+        else k_refine_final<T, false><<<nb, 256, 0, st>>>(G.dg, xk, xm, D[0], D[1], D[2], 0.f, (T*)xt_tiled);
     });
     CTR_CUDA_TRY(cudaGetLastError());
     return CTR_OK;

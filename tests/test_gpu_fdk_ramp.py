@@ -17,9 +17,9 @@ def test_fdk_row_lengths(nu, oracle_built):
     import gpu_b200
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
-    cfg = dict(nx=10, ny=10, nz=6, nu=nu, nv=7, nviews=3, vx=1.0, du=24.0 / nu, dso=1000.0, dod=-500.0)
+    cfg = dict(nx=10, ny=10, nz=6, nu=nu, nv=7, nviews=3, vx=1.0, du=1.6, dso=1000.0, dod=-500.0)
     if nu > 1000:
-        cfg.update(nv=3, nviews=1, nz=2)
+        cfg.update(nv=5, nviews=1, nz=2)
     g = gpu_b200.Geometry(ctr_desc(cfg))
     d = og_desc_xyz(cfg)
     o = oracle_built.Oracle(d)
