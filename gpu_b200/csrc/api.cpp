@@ -158,7 +158,12 @@ extern "C" ctr_status ctr_forward(const ctr_geometry* geom, const void* vol, ctr
     CTR_TRY(check_views(g, v0, n));
     FpArgs a{};
     a.vol = vol; a.vol_dtype = vdt; a.view0 = v0; a.nview = n; a.kind = FP_FORWARD; a.out = sino; a.out_dtype = sdt;
-    return forward_chunks(g, a, S(stream));
+    cudaStream_t st = S(stream);
+    void* scratch = forward_zcol_fits(*g, vdt, n) ? pool_alloc(g, forward_zcol_bytes(*g, vdt), st) : nullptr;
+    if (!scratch) return forward_chunks(g, a, st);
+    const ctr_status r = forward_zcol(*g, vol, vdt, scratch, sino, sdt, v0, n, st);
+    pool_free(scratch, st);
+    return r;
 }
 
 extern "C" ctr_status ctr_backproject(const ctr_geometry* geom, const float* sino, int v0, int n, void* vol,

@@ -92,6 +92,11 @@ struct Geometry {
     void* d_fgp = nullptr; size_t fgp_bytes = 0;       // 9 dual arrays
     float* d_fdk = nullptr; size_t fdk_cap = 0;
     void* d_tiled = nullptr; size_t tiled_bytes = 0;   // tiled copy for CTR_SART_TILED
+    // Scratch of one call (ctr_forward's copy of the volume), stream-ordered, so
+    // that calls on other streams and threads have their own.  The pool keeps
+    // at most about one FP32 volume between calls and goes with the geometry.
+    cudaMemPool_t pool = nullptr;
+    bool pool_tried = false;
     float* d_ramp = nullptr;                           // 2R-1 taps
     // slab geometries of the one-GPU slab SART (ctr_sart_pass_slabs), built on first use,
     // with a stream per slab and the events that order them around the combination
@@ -134,6 +139,10 @@ ctr_status ensure_fgp(Geometry* g, size_t bytes);
 // FGP workspace: three sets of the three duals in the storage type
 inline size_t fgp_workspace_bytes(long long V, ctr_dtype dt) { return (size_t)V * 9 * dtype_size(dt); }
 ctr_status ensure_tiled(Geometry* g, size_t bytes);
+// bytes of the geometry's pool on stream st, or NULL (no memory, or st is being
+// captured: the caller then takes a path without scratch); pool_free returns it
+void* pool_alloc(Geometry* g, size_t bytes, cudaStream_t st);
+void pool_free(void* p, cudaStream_t st);
 ctr_status check_device_errors(Geometry* g, cudaStream_t st);
 
 // ---- kernel launchers (implemented in the .cu files) ----
@@ -205,6 +214,14 @@ struct __align__(16) AdjRay {
 ctr_status launch_ray_prep(const Geometry& g, const float* y, int view0, int nview, AdjRay* rays,
                            cudaStream_t st);
 
+// Ray sums of views [view0, view0 + nview) into out, on a z-column copy of vol
+// made in scratch (forward_zcol_bytes; zcol.cu): the general projector's results,
+// bit for bit.  forward_zcol_fits: the geometry has such a path and the call is
+// large enough for it.
+bool forward_zcol_fits(const Geometry& g, ctr_dtype vdt, int nview);
+size_t forward_zcol_bytes(const Geometry& g, ctr_dtype vdt);
+ctr_status forward_zcol(const Geometry& g, const void* vol, ctr_dtype vdt, void* scratch, void* out, ctr_dtype out_dt,
+                        int view0, int nview, cudaStream_t st);
 // The matched adjoint as a z-column gather (zcol_adj.cu): views [view0,
 // view0 + nview) of y into vol.  ws: adj_record_bytes(g, nview) of scratch.
 // For fast_exit geometries with FP32 entry, the tetrahedron beam excepted.

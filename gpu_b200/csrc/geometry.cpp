@@ -102,6 +102,46 @@ ctr_status ensure_tiled(Geometry* g, size_t bytes)
     return CTR_OK;
 }
 
+// The geometry's pool, created by the first call that asks for it; nullptr where
+// the device has none.
+static cudaMemPool_t scratch_pool(Geometry* g)
+{
+    static std::mutex m;
+    std::lock_guard<std::mutex> lock(m);
+    if (!g->pool && !g->pool_tried) {
+        g->pool_tried = true;
+        cudaMemPoolProps pp{};
+        pp.allocType = cudaMemAllocationTypePinned;
+        pp.location.type = cudaMemLocationTypeDevice;
+        pp.location.id = g->device;
+        if (cudaMemPoolCreate(&g->pool, &pp) == cudaSuccess) {
+            uint64_t keep = (uint64_t)g->nvox() * sizeof(float) + (64u << 20);   // the pool's granularity
+            cudaMemPoolSetAttribute(g->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        } else {
+            g->pool = nullptr;
+        }
+        cudaGetLastError();
+    }
+    return g->pool;
+}
+
+void* pool_alloc(Geometry* g, size_t bytes, cudaStream_t st)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    void* p = nullptr;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+        const cudaMemPool_t pool = scratch_pool(g);
+        if (pool && cudaMallocFromPoolAsync(&p, bytes, pool, st) == cudaSuccess) return p;
+    }
+    cudaGetLastError();
+    return nullptr;
+}
+
+void pool_free(void* p, cudaStream_t st)
+{
+    if (p) cudaFreeAsync(p, st);
+}
+
 ctr_status check_device_errors(Geometry* g, cudaStream_t st)
 {
     unsigned h = 0;
@@ -489,6 +529,7 @@ extern "C" ctr_status ctr_geometry_destroy(ctr_geometry* geom)
     cudaFree(g->d_fgp);
     cudaFree(g->d_fdk);
     cudaFree(g->d_tiled);
+    if (g->pool) cudaMemPoolDestroy(g->pool);
     cudaFree(g->d_ramp);
     cudaFree(g->d_parts);
     if (g->split_geom) ctr_geometry_destroy(reinterpret_cast<ctr_geometry*>(g->split_geom));

@@ -1,21 +1,19 @@
 // zcol.cuh -- device parts shared by the z-column kernels (zcol_fp.cuh,
-// zcol_bp.cu).
+// zcol_adj.cu).
 //
-// The volume is held z-fastest, vol[(j*nx + i)*nz + k]: a "z-column" per
-// voxel column.  For a circular orbit the in-plane part of a ray depends only
-// on the view and the detector column, so the 32 lanes of a warp take 32 rows
-// of one detector column (projector) or 32 voxels of one z-column
-// (backprojectors): everything in-plane -- which voxel columns a ray crosses
-// and at which alphas, which detector columns cross a voxel column -- is the
-// same for the whole warp and is worked out once, and the lanes' voxels and
-// ray records lie next to each other in memory.
+// A z-column is the nz voxels over one (i, j).  For a circular orbit the
+// in-plane part of a ray depends only on the view and the detector column, so
+// the 32 lanes of a warp take 32 rows of one detector column (projector) or 32
+// voxels of one z-column (adjoint): everything in-plane -- which voxel columns a
+// ray crosses and at which alphas, which detector columns cross a voxel column
+// -- is the same for the whole warp and is worked out once, and the lanes'
+// voxels (in a z-fastest copy, for the projector) or ray records lie next to
+// each other.
 #pragma once
 
 #include "ctr_device.cuh"
 
 namespace ctr {
-
-__host__ __device__ inline long long zcol_count(const DevGeom& g) { return (long long)g.Z * g.M * g.N; }
 
 // floor of the position along an axis at parameter a, as a plane index (the
 // projector's pos_floor).

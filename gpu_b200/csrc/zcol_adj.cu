@@ -212,7 +212,7 @@ k_adj_cols(const __grid_constant__ DevGeom g, VT* __restrict__ vol, const AdjRec
             if (nrun == 0) continue;
             const float a0 = __fmaf_rn(c.mlo, zs0, z0), a1 = __fmaf_rn(c.mhi, zs0, z0);
             const float b0 = __fmaf_rn(c.mlo, zs1, z1), b1 = __fmaf_rn(c.mhi, zs1, z1);
-            const int vlo = max(__float2int_ru(__fmaf_rn(fminf(a0, a1), g.inv_dv, c.row_lo)), 0);
+            const int vlo = min(max(__float2int_ru(__fmaf_rn(fminf(a0, a1), g.inv_dv, c.row_lo)), 0), ZP);
             const int vhi = min(__float2int_rd(__fmaf_rn(fmaxf(b0, b1), g.inv_dv, c.row_hi)), ZP - 1);
             const int nrows = k < g.Z ? max(vhi - vlo + 1, 0) : 0;
             const int wrows = __reduce_max_sync(0xffffffffu, nrows);
