@@ -19,7 +19,9 @@
 //
 // k_backproject: the SART update (command 1) and the reference's command 0,
 // with the reference BP's geometric chords, FOV mask and thresholds.
-// k_adjoint: the exact adjoint of the forward projector.  Each ray record
+// k_adjoint: the exact adjoint of the forward projector, for the geometries the
+// z-column gather (zcol_adj.cu) does not cover (the tetrahedron beam, FP64 entry,
+// volumes that touch the detector plane).  Each ray record
 // carries the alpha interval, start voxel and parallel axes of the forward
 // traversal, and the chord of a voxel is taken over the traversal's own cell
 // intervals: the start cell opens at -inf, cells behind the start are never

@@ -1,0 +1,48 @@
+"""The z-column adjoint at the edges of its tiles: volumes one voxel short of,
+at and past 8 x 4 columns and 32 slices, a single voxel, detector columns much
+finer than a voxel (runs longer than the four a column keeps) and coarser,
+steep cones, accumulation, 16-bit volumes.  Against the oracle's scatter of the
+projector's own segments in FP64, to float rounding (as the parity test)."""
+import numpy as np
+import pytest
+
+from scan_configs import ctr_desc, og_desc_xyz
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def scan(nx, ny, nz, **kw):
+    return dict(dict(nx=nx, ny=ny, nz=nz, nu=29, nv=23, nviews=9, vx=1.0, du=1.3, dso=1000.0, dod=-500.0), **kw)
+
+
+SCANS = {
+    "8x4x32": scan(8, 4, 32), "9x5x33": scan(9, 5, 33, initial_angle=1.0), "7x3x31": scan(7, 3, 31),
+    "one": scan(1, 1, 1, du=0.2), "17x6x65": scan(17, 6, 65, nv=60), "slice": scan(24, 20, 1, nv=5),
+    "fine": scan(9, 8, 6, nu=130, nv=70, du=0.19), "coarse": scan(30, 29, 20, nu=9, nv=7, du=7.0),
+    "steep": scan(12, 10, 70, nu=24, nv=90, du=1.4, dso=30.0, dod=-30.0, initial_angle=3.0),
+}
+
+
+@pytest.mark.parametrize("name", sorted(SCANS))
+def test_adjoint_tile_edges(name, oracle_built):
+    import gpu_b200
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    cfg = SCANS[name]
+    g = gpu_b200.Geometry(ctr_desc(cfg))
+    o = oracle_built.Oracle(og_desc_xyz(cfg))
+    y = np.random.default_rng(3).standard_normal((cfg["nviews"],) + o.view_shape).astype(np.float32)
+    ref = o.adjoint(y)
+    dy = torch.from_numpy(y).cuda()
+    vol = torch.full(o.vol_shape, 7.0, device="cuda")
+    g.backproject(dy, vol)                                     # overwrites
+    got = vol.cpu().numpy().astype(np.float64)
+    top = np.abs(ref).max()
+    assert top > 0
+    assert np.all(np.abs(got - ref) <= 1.2e-7 * np.abs(ref) + 1e-12 * top)
+    g.backproject(dy, vol, flags=gpu_b200.BP_ACCUMULATE)       # one rounding of the sum
+    assert np.all(np.abs(vol.cpu().numpy() - 2.0 * got) <= 2.4e-7 * np.abs(ref) + 1e-12 * top)
+    half = torch.zeros(o.vol_shape, device="cuda", dtype=torch.bfloat16)
+    g.backproject(dy, half)
+    assert torch.equal(half.cpu(), torch.from_numpy(got.astype(np.float32)).to(torch.bfloat16))
