@@ -4,7 +4,7 @@
 // shared memory over a batch of views.  Per view each lane works out one
 // column's in-plane setup (vox_col); then the warp goes through its columns
 // with a lane per voxel: candidate rows, the two z alphas of a (voxel, row)
-// pair, and per detector column of the run one 16-byte record, the overlap
+// pair, and per detector column of the run one 8-byte record, the overlap
 // of two alpha intervals, and one FP64 multiply-add.  Chord = d12 x overlap in
 // the projector's own float alphas, so every (voxel, ray) chord is the
 // projector's Siddon segment bit for bit.
@@ -19,20 +19,22 @@
 // irregular rays with the traversal's own cell intervals (AdjRay).  No
 // atomics; every sum has a fixed order.
 //
-// Bound by issue (about 10 instructions a pair).  The form it replaces, which
+// Bound by load latency and issue (half the slots): a row's records are loaded
+// a row ahead.  The form it replaces, which
 // tested every candidate pair against the traversal record in 32 bytes, took
 // 0.59 ms a view of 256^3 voxels and 384^2 rays, records included; this one
-// takes 0.15 ms.
+// takes 0.14 ms (0.15 with 16-byte records and no load ahead).
 #include "fp_kernels.cuh"
 #include "zcol_bp.cuh"
 
 namespace ctr {
 
-struct __align__(16) AdjRec {
-    double y;     // the detector value
-    float d12;    // the ray's length source - pixel; 0: no regular chord
-    float irr;    // 1: an irregular ray, its traversal in the AdjRay array
+// A ray's record: the detector value, and its length source - pixel; 0: no
+// chord; -0: an irregular ray, its traversal in the AdjRay array.
+struct __align__(8) AdjRec {
+    float y, d12;
 };
+__device__ __forceinline__ bool irregular(const AdjRec& r) { return __float_as_uint(r.d12) == 0x80000000u; }
 
 // Records of views [view0, view0 + gridDim.z), [view][u][v].  A block of 32
 // columns x 8 rows; the records leave through shared memory so that the
@@ -56,9 +58,8 @@ k_adj_prep(const __grid_constant__ DevGeom g, const float* __restrict__ y, int v
     const float2 sc = g.trig[view0 + w];
     const RayInit r = ray_init(g, sc.x, sc.y, u, v);
     AdjRec rec;
-    rec.y = (double)yt[cu][rv];
+    rec.y = yt[cu][rv];
     rec.d12 = 0.0f;
-    rec.irr = 0.0f;
     if (r.hit) {
         // regular: the start voxel holds the entry (its entry planes at or
         // before amin, its exit planes at or after), and a parallel axis
@@ -85,7 +86,7 @@ k_adj_prep(const __grid_constant__ DevGeom g, const float* __restrict__ y, int v
             a.f = make_float4(yt[cu][rv], rr.d12, rr.a_lo, rr.a_hi);
             a.i = make_int4(rr.vi0, rr.vj0, rr.vk0, rr.par);
             full[w * P + (long long)u * g.ZP + v] = a;
-            rec.irr = 1.0f;
+            rec.d12 = -0.0f;
             marks[(long long)w * g.R + u] = 1;
         }
     }
@@ -156,7 +157,7 @@ static __device__ __noinline__ double irregular_sum(const DevGeom& g, const VoxC
         const float ay0 = fm(fs(ylo, ct.z), ct.w), ay1 = fm(fs(yhi, ct.z), ct.w);
         for (int vv = vlo; vv <= vhi; ++vv) {
             const long long p = (long long)uu * g.ZP + vv;
-            if (rw[p].irr == 0.0f) continue;
+            if (!irregular(rw[p])) continue;
             const AdjRay rec = fw[p];
             const float2 rt = g.rowt[vv];
             const float az0 = fm(fs(z0, rt.x), rt.y), az1 = fm(fs(z1, rt.x), rt.y);
@@ -176,7 +177,7 @@ static __device__ __noinline__ double irregular_sum(const DevGeom& g, const VoxC
 }
 
 template <typename VT>
-__global__ void __launch_bounds__(32 * AC_WARPS, 4)
+__global__ void __launch_bounds__(32 * AC_WARPS, 5)
 k_adj_cols(const __grid_constant__ DevGeom g, VT* __restrict__ vol, const AdjRec* __restrict__ recs,
            const AdjRay* __restrict__ full, const unsigned char* __restrict__ marks, int view0, int nview, int accumulate)
 {
@@ -225,33 +226,37 @@ k_adj_cols(const __grid_constant__ DevGeom g, VT* __restrict__ vol, const AdjRec
                 float2 iv[NQ];
 #pragma unroll
                 for (int t = 0; t < NQ; ++t) iv[t] = c.r[t];
-                for (int r = 0; r < wrows; ++r) {
+                // a row's records and row constants, loaded one row ahead
+                float2 rec[NQ], rt;
+                auto load = [&](int r) {
                     const int vv = min(vlo + r, ZP - 1);
-                    const bool on = r < nrows;
-                    const float2 rt = __ldg(g.rowt + vv);
-                    const float az0 = fm(fs(z0, rt.x), rt.y), az1 = fm(fs(z1, rt.x), rt.y);
-                    const float zl = fminf(az0, az1), zh = on ? fmaxf(az0, az1) : -1.0f;
-                    const float4* __restrict__ pr = reinterpret_cast<const float4*>(rc + vv);
+                    const float2* __restrict__ pr = reinterpret_cast<const float2*>(rc + vv);
 #pragma unroll
-                    for (int t = 0; t < NQ; ++t) {
-                        const float4 rec = __ldg(pr + (long long)t * ZP);
-                        const float temp = fm(rec.z, fs(fminf(iv[t].y, zh), fmaxf(iv[t].x, zl)));
-                        if (temp > 0.0f)
-                            acc = __fma_rn((double)temp,
-                                           __hiloint2double(__float_as_int(rec.y), __float_as_int(rec.x)), acc);
+                    for (int t = 0; t < NQ; ++t) rec[t] = __ldg(pr + (long long)t * ZP);
+                    rt = __ldg(g.rowt + vv);
+                };
+                load(0);
+                for (int r = 0; r < wrows; ++r) {
+                    float2 now[NQ];
+#pragma unroll
+                    for (int t = 0; t < NQ; ++t) now[t] = rec[t];
+                    const float az0 = fm(fs(z0, rt.x), rt.y), az1 = fm(fs(z1, rt.x), rt.y);
+                    load(r + 1);
+                    const float zl = fminf(az0, az1), zh = r < nrows ? fmaxf(az0, az1) : -1.0f;
+                    auto pair = [&](const float2& a, const float2& w2) {
+                        const float temp = fm(w2.y, fs(fminf(a.y, zh), fmaxf(a.x, zl)));
+                        if (temp > 0.0f) acc = __fma_rn((double)temp, (double)w2.x, acc);
+                    };
+#pragma unroll
+                    for (int t = 0; t < NQ; ++t) pair(iv[t], now[t]);
+                    if (NQ == ZC_RUN) {   // runs longer than the column keeps
+                        const int ii = i0 + (q % AC_X), jj = j0 + q / AC_X;
+                        const float2* __restrict__ pr = reinterpret_cast<const float2*>(rc + min(vlo + r, ZP - 1));
+                        for (int t = ZC_RUN; t < nrun; ++t)
+                            pair(col_interval(__ldg(g.colt + (long long)view * g.R + c.ua + t), __ldg(g.px + ii + 1),
+                                              __ldg(g.px + ii + 2), __ldg(g.py + jj + 1), __ldg(g.py + jj + 2)),
+                                 __ldg(pr + (long long)t * ZP));
                     }
-                    if (NQ == ZC_RUN)
-                        for (int t = ZC_RUN; t < nrun; ++t) {
-                            const int ii = i0 + (q % AC_X), jj = j0 + q / AC_X;
-                            const float2 a = col_interval(__ldg(g.colt + (long long)view * g.R + c.ua + t),
-                                                          __ldg(g.px + ii + 1), __ldg(g.px + ii + 2),
-                                                          __ldg(g.py + jj + 1), __ldg(g.py + jj + 2));
-                            const float4 rec = __ldg(pr + (long long)t * ZP);
-                            const float temp = fm(rec.z, fs(fminf(a.y, zh), fmaxf(a.x, zl)));
-                            if (temp > 0.0f)
-                                acc = __fma_rn((double)temp,
-                                               __hiloint2double(__float_as_int(rec.y), __float_as_int(rec.x)), acc);
-                        }
                 }
             };
             if (nrun <= 2) {
