@@ -301,9 +301,9 @@ ctr_status launch_adjoint_cols(const Geometry& G, const float* y, int view0, int
     const DevGeom& g = G.dg;
     if (nview <= 0) return CTR_OK;
     const size_t n = (size_t)g.R * g.ZP * nview;
-    AdjRec* recs = (AdjRec*)ws;
-    AdjRay* full = (AdjRay*)(recs + n);
-    unsigned char* marks = (unsigned char*)(full + n);
+    AdjRay* full = (AdjRay*)ws;   // first: 16-byte aligned for any number of rays
+    AdjRec* recs = (AdjRec*)(full + n);
+    unsigned char* marks = (unsigned char*)(recs + n);
     CTR_CUDA_TRY(cudaMemsetAsync(marks, 0, (size_t)g.R * nview, st));
     k_adj_prep<<<dim3((g.R + AP_COLS - 1) / AP_COLS, (g.ZP + AP_ROWS - 1) / AP_ROWS, nview), AP_ROWS * AP_COLS, 0, st>>>(
         g, y, view0, recs, full, marks);

@@ -20,6 +20,9 @@ SCANS = {
     "8x4x32": scan(8, 4, 32), "9x5x33": scan(9, 5, 33, initial_angle=1.0), "7x3x31": scan(7, 3, 31),
     "one": scan(1, 1, 1, du=0.2), "17x6x65": scan(17, 6, 65, nv=60), "slice": scan(24, 20, 1, nv=5),
     "fine": scan(9, 8, 6, nu=130, nv=70, du=0.19), "coarse": scan(30, 29, 20, nu=9, nv=7, du=7.0),
+    # an odd number of rays in a batch, axis-parallel and on-plane rays among them
+    "odd_rays": scan(12, 12, 12, nu=17, nv=13, nviews=7, du=1.6),
+    "odd_planes": scan(11, 12, 11, nu=17, nv=13, nviews=1, du=1.5),
     "steep": scan(12, 10, 70, nu=24, nv=90, du=1.4, dso=30.0, dod=-30.0, initial_angle=3.0),
 }
 
