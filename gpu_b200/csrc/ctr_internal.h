@@ -97,7 +97,7 @@ struct Geometry {
     // at most about one FP32 volume between calls and goes with the geometry.
     cudaMemPool_t pool = nullptr;
     bool pool_tried = false;
-    float* d_ramp = nullptr;                           // 2R-1 taps
+    float* d_ramp = nullptr;                           // FDK's filter tables (fdk.cu): k_ramp_fft's, or 2R-1 taps
     // slab geometries of the one-GPU slab SART (ctr_sart_pass_slabs), built on first use,
     // with a stream per slab and the events that order them around the combination
     std::vector<Geometry*> slab_geoms;

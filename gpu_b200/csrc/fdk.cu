@@ -96,56 +96,68 @@ k_ramp(const float* __restrict__ in, float* __restrict__ out, const float* __res
     }
 }
 
-// ---- weight and ramp of two detector rows by FFT
+// ---- weight and ramp of a detector row by FFT
 //
-// The taps are real and even, so their spectrum is real: a row pair a + i b
-// stays a pair through FFT, product and inverse FFT, and no unpacking is
-// needed.  n = a power of two >= 2R - 1 points; Stockham passes of radix 8
+// A row of R values is n = a power of two >= 2R - 1 real points, transformed in
+// FP64 as n/2 complex ones (even + i odd points): Stockham passes of radix 8
 // (radix 4 or 2 last), 8 points a thread, exchanged through one padded
-// shared-memory buffer.  The first pass reads the rows (weighted on the way,
-// zero beyond R), the last inverse pass writes them.
-// 1024-point rows: 15 n log2 n = 0.34 MFLOP a pair instead of the Toeplitz
-// product's 4.2 M multiply-adds; bound by shared memory (7 exchanges).
-// 1024 views x 768 rows of 1024: 12.3 ms, weight included (Toeplitz 37.6 ms and
-// the weight pass 3.3 ms).
-static constexpr int kFftMost = 8192;   // 1024 threads, 147 KB of shared memory
+// shared-memory buffer.  The first pass reads the row (weighted on the way with
+// k_fdk_weight's operations, zero beyond R); the inverse's first pass separates
+// the two interleaved spectra, multiplies by the taps' spectrum (real: the taps
+// are even) and joins them again; its last pass writes the row.  Short rows
+// share a block.
+//
+// FP64 because the ramp removes what a smooth row is made of, low frequencies:
+// an FP32 transform's error follows the row's largest values and is several
+// times the direct sum's.  A row alone because two rows as the real and
+// imaginary part of one transform share their rounding error and every NaN.  A
+// row with a non-finite value is summed directly (its transform would turn one
+// Inf into NaN everywhere), with k_ramp's operations.
+//
+// Bound by latency and shared memory (8 exchanges of 16 KB for 1024 values),
+// 24 warps an SM (78 registers).  256 views x 768 rows of 1024: 4.0 ms, weight
+// included; 4.4 ms at 16 warps; FP32 pairs of rows 3.2 ms; the Toeplitz product
+// and the weight pass 10.4 ms.  64 rows of 64, 360 views: 45, 52 and 63 us.
+static constexpr int kFftMost = 8192;     // 512 threads, 74 KB of shared memory
+static constexpr int kFftBlock = 128;     // threads of a block of short rows
 
 __device__ __forceinline__ int fft_pad(int i) { return i + (i >> 3); }
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 cmul(float2 a, float2 b)
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 cmul(double2 a, double2 b)
 {
-    return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
+    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
 }
 // i*a (inverse) or -i*a (forward)
-template <bool INV> __device__ __forceinline__ float2 crot(float2 a)
+template <bool INV> __device__ __forceinline__ double2 crot(double2 a)
 {
-    return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+    return INV ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x);
 }
-template <bool INV> __device__ __forceinline__ void fft2(float2& a, float2& b)
+__device__ __forceinline__ void fft2(double2& a, double2& b)
 {
-    const float2 t = csub(a, b);
+    const double2 t = csub(a, b);
     a = cadd(a, b);
     b = t;
 }
-template <bool INV> __device__ __forceinline__ void fft4(float2* v)   // in order
+template <bool INV> __device__ __forceinline__ void fft4(double2* v)   // in order
 {
-    float2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]), c = cadd(v[1], v[3]), d = crot<INV>(csub(v[1], v[3]));
+    const double2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]), c = cadd(v[1], v[3]), d = crot<INV>(csub(v[1], v[3]));
     v[0] = cadd(a, c);
     v[1] = cadd(b, d);
     v[2] = csub(a, c);
     v[3] = csub(b, d);
 }
-template <bool INV> __device__ __forceinline__ void fft8(float2* v)   // in order
+template <bool INV> __device__ __forceinline__ void fft8(double2* v)   // in order
 {
-    const float h = 0.70710678118654752440f;
-    float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+    const double h = 0.70710678118654752440;
+    double2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
     fft4<INV>(e);
     fft4<INV>(o);
-    const float2 w1 = INV ? make_float2(h, h) : make_float2(h, -h), w3 = INV ? make_float2(-h, h) : make_float2(-h, -h);
-    o[1] = cmul(o[1], w1);
+    // o1 exp(-+i pi/4) and o3 exp(-+3i pi/4)
+    const double2 r1 = crot<INV>(o[1]), r3 = crot<INV>(o[3]);
+    o[1] = make_double2(h * (o[1].x + r1.x), h * (o[1].y + r1.y));
     o[2] = crot<INV>(o[2]);
-    o[3] = cmul(o[3], w3);
+    o[3] = make_double2(h * (r3.x - o[3].x), h * (r3.y - o[3].y));
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
         v[t] = cadd(e[t], o[t]);
@@ -154,111 +166,130 @@ template <bool INV> __device__ __forceinline__ void fft8(float2* v)   // in orde
 }
 
 // One pass of radix RX over n points whose sub-transforms have length ns:
-// thread index j of n / RX reads points j + m n/RX and writes
+// thread index j of n / RX holds points j + m n/RX; the results go to
 // (j/ns) ns RX + j%ns + m ns.  tw[t] = exp(-2 pi i t / n).
 template <int RX, bool INV>
-__device__ __forceinline__ void fft_radix(float2* v, int j, int ns, int n, const float2* __restrict__ tw)
+__device__ __forceinline__ void fft_radix(double2* v, int j, int ns, int n, const double2* __restrict__ tw)
 {
     if (ns > 1) {
-        const int k = j & (ns - 1), s = n / (ns * RX);
+        double2 w[8];   // powers of the butterfly's root: one load
+        w[1] = __ldg(tw + (j & (ns - 1)) * (n / (ns * RX)));
+        if (INV) w[1].y = -w[1].y;
 #pragma unroll
-        for (int m = 1; m < RX; ++m) {
-            float2 w = __ldg(tw + k * m * s);
-            if (INV) w.y = -w.y;
-            v[m] = cmul(v[m], w);
-        }
+        for (int m = 2; m < RX; ++m) w[m] = cmul(w[m >> 1], w[m - (m >> 1)]);
+#pragma unroll
+        for (int m = 1; m < RX; ++m) v[m] = cmul(v[m], w[m]);
     }
     if (RX == 8) fft8<INV>(v);
     else if (RX == 4) fft4<INV>(v);
-    else fft2<INV>(v[0], v[1]);
+    else fft2(v[0], v[1]);
 }
 
-// The passes of one direction over the thread's 8 points.  get(i) yields
-// point i of the first pass, put(i, v) takes point i of the last; in between
-// the points go through sh.  The sub-transform lengths are 1, 8, 64, ...; a
-// last pass of radix 2 or 4 does 4 or 2 of them per thread.
+// The passes of one direction over the 8 points of thread j of a row.  get(i)
+// yields point i of the first pass, put(i, v) takes point i of the last; in
+// between the points go through sh.  The forward's get does not read sh, the
+// inverse's put does not write it.  The sub-transform lengths are 1, 8, 64, ...; a
+// last pass of radix 2 or 4 does 4 or 2 butterflies a thread.
 template <bool INV, typename G, typename P>
-__device__ __forceinline__ void fft_passes(float2* sh, int n, int log2n, const float2* __restrict__ tw, G get, P put)
+__device__ __forceinline__ void fft_passes(double2* sh, int j, int n, int log2n, const double2* __restrict__ tw, G get, P put)
 {
-    const int j = threadIdx.x, T = n >> 3;
-    float2 v[8];
+    const int T = n >> 3;
+    double2 v[8];
     int ns = 1;
     for (int left = log2n; left > 0;) {
         const bool first = ns == 1;
         const int lr = left >= 3 ? 3 : left;
         const bool last = left == lr;
-        if (!first) __syncthreads();   // the previous pass's stores
+        const bool reads = INV || !first, writes = !INV || !last;   // of sh
+        if (reads) __syncthreads();   // the previous pass's stores
         if (lr == 3) {
 #pragma unroll
             for (int m = 0; m < 8; ++m) v[m] = first ? get(j + m * T) : sh[fft_pad(j + m * T)];
             fft_radix<8, INV>(v, j, ns, n, tw);
-            if (!first) __syncthreads();   // every load done
-            const int base = (j / ns) * ns * 8 + (j & (ns - 1));
+        } else {   // never the first pass: n >= 8
+            if (lr == 2) {
 #pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                if (last) put(base + m * ns, v[m]);
-                else sh[fft_pad(base + m * ns)] = v[m];
+                for (int q = 0; q < 8; ++q) v[q] = sh[fft_pad(j + (q >> 2) * T + (q & 3) * 2 * T)];
+                fft_radix<4, INV>(v, j, ns, n, tw);
+                fft_radix<4, INV>(v + 4, j + T, ns, n, tw);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = sh[fft_pad(j + (q >> 1) * T + (q & 1) * 4 * T)];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) fft_radix<2, INV>(v + 2 * h, j + h * T, ns, n, tw);
             }
-        } else if (lr == 2) {   // two radix-4 butterflies: j and j + T
+        }
+        if (reads && writes) __syncthreads();   // every load done
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int m = 0; m < 4; ++m) v[4 * h + m] = sh[fft_pad(j + h * T + m * 2 * T)];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int jj = j + h * T;
-                fft_radix<4, INV>(v + 4 * h, jj, ns, n, tw);
-#pragma unroll
-                for (int m = 0; m < 4; ++m) put((jj / ns) * ns * 4 + (jj & (ns - 1)) + m * ns, v[4 * h + m]);
-            }
-        } else {
-#pragma unroll
-            for (int h = 0; h < 4; ++h)
-#pragma unroll
-                for (int m = 0; m < 2; ++m) v[2 * h + m] = sh[fft_pad(j + h * T + m * 4 * T)];
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                const int jj = j + h * T;
-                fft_radix<2, INV>(v + 2 * h, jj, ns, n, tw);
-#pragma unroll
-                for (int m = 0; m < 2; ++m) put((jj / ns) * ns * 2 + (jj & (ns - 1)) + m * ns, v[2 * h + m]);
-            }
+        for (int q = 0; q < 8; ++q) {
+            const int jj = j + (q >> lr) * T, m = q & ((1 << lr) - 1);
+            const int at = ((jj & ~(ns - 1)) << lr) + (jj & (ns - 1)) + m * ns;
+            if (last) put(at, v[q]);
+            else sh[fft_pad(at)] = v[q];
         }
         ns <<= lr;
         left -= lr;
     }
 }
 
-// rows 2 blockIdx.x and 2 blockIdx.x + 1 of nrows rows of R values (row % ZP is
-// the detector row): out = ramp(weight * in).  n / 8 threads.  H[k] / n is the
-// taps' spectrum in sp.
-__global__ void __launch_bounds__(kFftMost / 8)
-k_ramp_fft(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ weight,
-           const float2* __restrict__ tw, const float* __restrict__ sp, int R, int ZP, long long nrows, int n, int log2n)
+// Tables of k_ramp_fft (fft_tables): N = n/2 roots exp(-2 pi i t / N); per k
+// of N the pair exp(-2 pi i k / n), (H[k] +- H[N-k]) / 2N; the weights' roots
+// [v][u]; R taps.
+struct FftTables {
+    const double2* tw;
+    const double2* un;
+    const float* root;
+    const float* taps;
+};
+
+// Rows of nrows rows of R values (row % ZP is the detector row): out = ramp(weight
+// * in).  A block takes blockDim.x / (N/8) rows.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == kFftBlock ? 6 : 1)
+k_ramp_fft(const float* __restrict__ in, float* __restrict__ out, const FftTables tb, float dso, int R, int ZP,
+           long long nrows, int N, int log2N)
 {
-    extern __shared__ float2 fsh[];
-    const long long r0 = 2LL * blockIdx.x;
-    const bool two = r0 + 1 < nrows;
-    const float* __restrict__ a = in + r0 * R;
-    const float* __restrict__ wa = weight + (r0 % ZP) * R;
-    const float* __restrict__ wb = weight + ((r0 + 1) % ZP) * R;
-    auto read = [&](int i) {
-        if (i >= R) return make_float2(0.0f, 0.0f);
-        return make_float2(__ldg(a + i) * __ldg(wa + i), two ? __ldg(a + R + i) * __ldg(wb + i) : 0.0f);
-    };
-    // the spectrum goes back through shared memory in order
-    fft_passes<false>(fsh, n, log2n, tw, read, [&](int i, float2 v) {
-        const float h = __ldg(sp + i);
-        fsh[n + (n >> 3) + fft_pad(i)] = make_float2(v.x * h, v.y * h);
-    });
+    extern __shared__ double2 fsh[];
+    __shared__ int bad[kFftBlock];   // rows with a non-finite value
+    const int T = N >> 3, rl = threadIdx.x / T, j = threadIdx.x - rl * T;
+    const long long row = (long long)blockIdx.x * (blockDim.x / T) + rl;
+    const bool live = row < nrows;
+    double2* const sh = fsh + (size_t)rl * (N + T);
+    const float* __restrict__ a = in + (live ? row : 0) * R;
+    const float* __restrict__ rt = tb.root + (live ? row % ZP : 0) * R;
+    if (j == 0) bad[rl] = 0;
     __syncthreads();
-    float* __restrict__ o = out + r0 * R;
-    fft_passes<true>(fsh, n, log2n, tw, [&](int i) { return fsh[n + (n >> 3) + fft_pad(i)]; }, [&](int i, float2 v) {
-        if (i < R) {
-            o[i] = v.x;
-            if (two) o[R + i] = v.y;
-        }
+    auto value = [&](int i) { return fdv(fm(__ldg(a + i), dso), __ldg(rt + i)); };   // kernel_FDK.cu:1-14
+    bool off = false;
+    fft_passes<false>(sh, j, N, log2N, tb.tw, [&](int i) {
+        float x = 0.0f, y = 0.0f;
+        if (live && 2 * i < R) x = value(2 * i);
+        if (live && 2 * i + 1 < R) y = value(2 * i + 1);
+        off |= !(fabsf(x) <= 3.402823466e38f) || !(fabsf(y) <= 3.402823466e38f);
+        return make_double2((double)x, (double)y);
+    }, [&](int i, double2 v) { sh[fft_pad(i)] = v; });
+    if (off) bad[rl] = 1;
+    // Z = E + iO, the spectra of the even and the odd points; with the taps'
+    // X[k] = E + W O, X[k+N] = E - W O become H[k] X[k], H[N-k] X[k+N]
+    float* __restrict__ o = out + (live ? row : 0) * R;
+    fft_passes<true>(sh, j, N, log2N, tb.tw, [&](int k) {
+        const double2 z = sh[fft_pad(k)], y = sh[fft_pad((N - k) & (N - 1))];
+        const double2 w = __ldg(tb.un + 2 * k), h = __ldg(tb.un + 2 * k + 1);
+        const double2 e = make_double2(0.5 * (z.x + y.x), 0.5 * (z.y - y.y));
+        const double2 od = make_double2(0.5 * (z.y + y.y), 0.5 * (y.x - z.x));
+        const double2 wo = cmul(w, od), we = cmul(make_double2(w.x, -w.y), e);
+        return make_double2(fma(h.x, z.x, h.y * (wo.x - we.y)), fma(h.x, z.y, h.y * (wo.y + we.x)));
+    }, [&](int i, double2 v) {
+        if (!live || bad[rl]) return;
+        if (2 * i < R) o[2 * i] = (float)v.x;
+        if (2 * i + 1 < R) o[2 * i + 1] = (float)v.y;
     });
+    if (live && bad[rl])
+        for (int u = j; u < R; u += T) {
+            float acc = 0.0f;
+            for (int m = 0; m < R; ++m) acc = fmaf(value(m), __ldg(tb.taps + abs(u - m)), acc);
+            o[u] = acc;
+        }
 }
 
 static constexpr int FB_BX = 32, FB_BY = 4, FB_K = 8;
@@ -371,7 +402,7 @@ k_fdk_bp(const __grid_constant__ DevGeom g, float* __restrict__ vol, const float
 }
 
 // h[n + R - 1], |n| < R, of the reference's padded-DFT ramp (FP64, as the oracle).
-static void ramp_taps(const ctr_geometry_desc& d, std::vector<float>& taps)
+static void ramp_taps(const ctr_geometry_desc& d, std::vector<double>& taps)
 {
     const int R = d.nu, P = 2 * R;
     const float DSO = d.dso, DOD = d.dod;
@@ -384,51 +415,74 @@ static void ramp_taps(const ctr_geometry_desc& d, std::vector<float>& taps)
         hv *= 0.5f;
         H[i] = hv;
     }
-    taps.assign(2 * R - 1, 0.f);
+    taps.assign(2 * R - 1, 0.0);
     std::vector<double> cosine(P);
     for (int m = 0; m < P; ++m) cosine[m] = std::cos(2.0 * M_PI * (double)m / (double)P);
     for (int n = 0; n <= R - 1; ++n) {
         double acc = 0.0;
         for (int i = 0, m = 0; i < P; ++i, m = m + n < P ? m + n : m + n - P) acc += (double)H[i] * cosine[m];   // m = i n mod P
-        taps[R - 1 + n] = taps[R - 1 - n] = (float)(acc / (double)P);
+        taps[R - 1 + n] = taps[R - 1 - n] = acc / (double)P;
     }
 }
 
-// Tables of k_ramp_fft, one allocation: n twiddles exp(-2 pi i t / n), the taps'
-// spectrum / n, the cosine weights [v][u] (kernel_FDK.cu:1-14).
+// The tables of k_ramp_fft, one allocation (G.d_ramp).
 static size_t fft_points(int R)
 {
-    size_t n = 8;
+    size_t n = 16;
     while (n < 2 * (size_t)R - 1) n <<= 1;
     return n;
 }
-static ctr_status fft_tables(Geometry& G, const std::vector<float>& taps)
+static FftTables fft_table_pointers(const Geometry& G, size_t N)
 {
-    const int R = G.desc.nu, ZP = G.dg.ZP;
-    const size_t n = fft_points(R);
-    std::vector<float> h(3 * n + (size_t)R * ZP);
-    std::vector<double> cosine(n);
+    FftTables t;
+    t.tw = reinterpret_cast<const double2*>(G.d_ramp);
+    t.un = t.tw + N;
+    t.root = reinterpret_cast<const float*>(t.un + 2 * N);
+    t.taps = t.root + (size_t)G.dg.R * G.dg.ZP;
+    return t;
+}
+static ctr_status fft_tables(Geometry& G, const std::vector<double>& taps)
+{
+    const DevGeom& g = G.dg;
+    const int R = g.R, ZP = g.ZP;
+    const size_t n = fft_points(R), N = n / 2;
+    std::vector<double> c(n), s(n), d(6 * N), H(N + 1);   // cos, sin(2 pi t / n); the FP64 tables; the spectrum / N
     for (size_t t = 0; t < n; ++t) {
         const double a = 2.0 * M_PI * (double)t / (double)n;
-        cosine[t] = std::cos(a);
-        h[2 * t] = (float)cosine[t];
-        h[2 * t + 1] = (float)-std::sin(a);
+        c[t] = std::cos(a);
+        s[t] = std::sin(a);
     }
-    for (size_t k = 0; k <= n / 2; ++k) {
+    for (size_t k = 0; k <= N; ++k) {
         double acc = taps[R - 1];
-        for (int m = 1; m < R; ++m) acc += 2.0 * (double)taps[R - 1 + m] * cosine[(k * (size_t)m) & (n - 1)];
-        h[2 * n + k] = h[2 * n + ((n - k) & (n - 1))] = (float)(acc / (double)n);
+        for (int m = 1; m < R; ++m) acc += 2.0 * taps[R - 1 + m] * c[(k * (size_t)m) & (n - 1)];
+        H[k] = acc / (double)N;
     }
-    const DevGeom& g = G.dg;
-    const double mag = (double)g.dso / ((double)g.dso - (double)g.dod);
-    for (int v = 0; v < ZP; ++v)
-        for (int u = 0; u < R; ++u) {
-            const double x2 = ((double)g.ymin + (double)u * g.du) * mag, x3 = ((double)g.zmin + (double)v * g.dv) * mag;
-            h[3 * n + (size_t)v * R + u] =
-                (float)((double)g.dso / std::sqrt((double)g.dso * g.dso + x2 * x2 + x3 * x3));
-        }
-    CTR_CUDA_TRY(cudaMalloc(&G.d_ramp, h.size() * sizeof(float)));
-    CTR_CUDA_TRY(cudaMemcpy(G.d_ramp, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
+    for (size_t k = 0; k < N; ++k) {
+        d[2 * k] = c[2 * k];
+        d[2 * k + 1] = -s[2 * k];
+        double* un = d.data() + 2 * N + 4 * k;
+        un[0] = c[k];
+        un[1] = -s[k];
+        un[2] = 0.5 * (H[k] + H[N - k]);
+        un[3] = 0.5 * (H[k] - H[N - k]);
+    }
+    // the weights' roots with k_fdk_weight's operations (float, each rounded), and the taps
+    std::vector<float> f((size_t)R * ZP + R);
+    const float dd = g.dso - g.dod, x1x1 = g.dso * g.dso;
+    std::vector<float> x2x2(R);
+    for (int u = 0; u < R; ++u) {
+        const float x2 = (g.ymin + (float)u * g.du) * g.dso / dd;
+        x2x2[u] = x2 * x2;
+        f[(size_t)R * ZP + u] = (float)taps[R - 1 + u];
+    }
+    for (int v = 0; v < ZP; ++v) {
+        const float x3 = (g.zmin + (float)v * g.dv) * g.dso / dd, x3x3 = x3 * x3;
+        for (int u = 0; u < R; ++u) f[(size_t)v * R + u] = std::sqrt((x1x1 + x2x2[u]) + x3x3);
+    }
+    const size_t db = d.size() * sizeof(double), fb = f.size() * sizeof(float);
+    CTR_CUDA_TRY(cudaMalloc(&G.d_ramp, db + fb));
+    CTR_CUDA_TRY(cudaMemcpy(G.d_ramp, d.data(), db, cudaMemcpyHostToDevice));
+    CTR_CUDA_TRY(cudaMemcpy((char*)G.d_ramp + db, f.data(), fb, cudaMemcpyHostToDevice));
     return CTR_OK;
 }
 
@@ -440,13 +494,14 @@ ctr_status launch_fdk(Geometry& G, const float* sino, float* vol, cudaStream_t s
     const size_t n = fft_points(g.R);
     const bool fft = n <= (size_t)kFftMost;
     if (!G.d_ramp) {
-        std::vector<float> taps;
+        std::vector<double> taps;
         ramp_taps(G.desc, taps);
         if (fft) {
             CTR_TRY(fft_tables(G, taps));
         } else {
-            CTR_CUDA_TRY(cudaMalloc(&G.d_ramp, taps.size() * sizeof(float)));
-            CTR_CUDA_TRY(cudaMemcpy(G.d_ramp, taps.data(), taps.size() * sizeof(float), cudaMemcpyHostToDevice));
+            const std::vector<float> h(taps.begin(), taps.end());
+            CTR_CUDA_TRY(cudaMalloc(&G.d_ramp, h.size() * sizeof(float)));
+            CTR_CUDA_TRY(cudaMemcpy(G.d_ramp, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
         }
     }
     const size_t need = (size_t)P * nv * (fft ? 1 : 2);
@@ -460,15 +515,19 @@ ctr_status launch_fdk(Geometry& G, const float* sino, float* vol, cudaStream_t s
     float* fsino = G.d_fdk;
     const long long nrows = (long long)nv * g.ZP;
     if (fft) {
-        int log2n = 0;
-        while ((1u << log2n) < n) ++log2n;
-        const size_t smem = 2 * (n + (n >> 3)) * sizeof(float2);
-        CTR_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(&k_ramp_fft),
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        const float2* tw = (const float2*)G.d_ramp;
-        const float* sp = G.d_ramp + 2 * n;
-        k_ramp_fft<<<(unsigned)((nrows + 1) / 2), (unsigned)(n / 8), smem, st>>>(sino, fsino, sp + n, tw, sp, g.R, g.ZP,
-                                                                                nrows, (int)n, log2n);
+        const int N = (int)(n / 2), T = N / 8, rows = std::max(1, kFftBlock / T);   // rows of a block
+        int log2N = 0;
+        while ((1 << log2N) < N) ++log2N;
+        const size_t smem = (size_t)rows * (N + T) * sizeof(double2);
+        const unsigned blocks = (unsigned)((nrows + rows - 1) / rows);
+        const FftTables tb = fft_table_pointers(G, N);
+        if (rows * T == kFftBlock) {
+            k_ramp_fft<kFftBlock><<<blocks, kFftBlock, smem, st>>>(sino, fsino, tb, g.dso, g.R, g.ZP, nrows, N, log2N);
+        } else {
+            CTR_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(&k_ramp_fft<kFftMost / 16>),
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
+            k_ramp_fft<kFftMost / 16><<<blocks, rows * T, smem, st>>>(sino, fsino, tb, g.dso, g.R, g.ZP, nrows, N, log2N);
+        }
     } else {
         float* wsino = G.d_fdk + (size_t)P * nv;
         for (int v0 = 0; v0 < nv; v0 += 65535) {

@@ -29,3 +29,62 @@ def test_fdk_row_lengths(nu, oracle_built):
     ref = o.fdk(b)
     assert np.abs(ref).max() > 0
     assert np.abs(vol.cpu().numpy() - ref).max() <= 1e-4 * np.abs(ref).max()
+
+
+def rows_scan(nu, nv):
+    """A thin column of voxels whose slices read every detector row, four slices a row."""
+    cfg = dict(nx=4, ny=4, nz=4 * nv, nu=nu, nv=nv, nviews=3, vx=0.25, du=1.5, dso=1000.0, dod=-500.0)
+    return cfg, og_desc_xyz(cfg)
+
+
+def both(cfg, o, b):
+    import gpu_b200
+    vol = torch.zeros(o.vol_shape, device="cuda")
+    gpu_b200.Geometry(ctr_desc(cfg)).fdk(torch.from_numpy(b).cuda(), vol)
+    return vol.cpu().numpy(), o.fdk(b)
+
+
+@pytest.mark.parametrize("nu,nv", [(16, 8), (100, 7), (1000, 8), (4097, 5)])
+def test_fdk_rows_are_filtered_alone(nu, nv, oracle_built):
+    """A detector row's values reach the voxels that read that row and no others: a NaN, an Inf, rows 1e4 times their
+    neighbours, rows of zeros, for an even and an odd number of rows.  The oracle's filter is a direct FP64 sum per
+    row.  Rows of a transform (nu <= 4096) come out correctly rounded but for rare ties, so voxels agree to the
+    backprojection's own rounding: 1e-6 of the largest among them."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    cfg, d = rows_scan(nu, nv)
+    o = oracle_built.Oracle(d)
+    rng = np.random.default_rng(nu)
+    b = rng.standard_normal((3,) + o.view_shape).astype(np.float32)
+    clean, ref = both(cfg, o, b)
+    tol = 1e-6 if nu <= 4096 else 1e-5   # a Toeplitz product of 4097 FP32 terms
+    assert np.abs(clean - ref).max() <= tol * np.abs(ref).max()
+    for bad in (np.nan, np.inf, -np.inf):
+        for w, v in ((1, 2), (2, nv - 1), (0, 0)):
+            c = b.copy()
+            c[w, v, nu // 3] = bad
+            got, want = both(cfg, o, c)
+            hit = ~np.isfinite(want)
+            assert hit.any() and not hit.all()
+            assert np.array_equal(~np.isfinite(got), hit), (bad, w, v)
+            assert np.array_equal(got[~hit], clean[~hit]), (bad, w, v)
+    strong = np.zeros(b.shape, bool)
+    strong[:, np.arange(nv) % 4 % 3 == 0] = True    # rows s w w s s w w s ...
+    only = both(cfg, o, np.where(strong, b, np.float32(0)))
+    quiet = only[1] == 0.0                           # voxels between two weak rows
+    assert quiet.any() and not quiet.all()
+    assert not only[0][quiet].any()
+    got, want = both(cfg, o, np.where(strong, np.float32(1e4), np.float32(1)) * b)
+    assert np.abs(got - want)[quiet].max() <= tol * np.abs(want[quiet]).max()
+
+
+def test_fdk_smooth_rows(oracle_built):
+    """Rows that are nearly constant: what the ramp leaves is small against the row, and is still right to FP32."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    cfg, d = rows_scan(1024, 6)
+    o = oracle_built.Oracle(d)
+    u = np.linspace(-1, 1, 1024)
+    b = (5.0 + np.exp(-u ** 2) + 0.01 * np.cos(40 * u))[None, None, :] * (1.0 + 0.1 * np.arange(6))[None, :, None]
+    got, want = both(cfg, o, np.repeat(b, 3, 0).astype(np.float32))
+    assert np.abs(got - want).max() <= 1e-6 * np.abs(want).max()
