@@ -188,7 +188,8 @@ extern "C" ctr_status ctr_backproject(const ctr_geometry* geom, const float* sin
     // test is one comparison (no chord is cut short at the exit) with FP32
     // entry; the other geometries and the masked form keep the general kernels.
     if (!masked && g->dg.fast_exit && !g->dg.entry64 && g->dg.ct_style != 3) {
-        CTR_TRY(ensure_rays(g, adj_record_bytes(g->dg, std::min(batch, n))));
+        // for a whole batch whatever n is: the workspace of a captured call is not replaced by a longer one
+        CTR_TRY(ensure_rays(g, adj_record_bytes(g->dg, batch)));
         for (int c = 0; c < n; c += batch) {
             const int cnt = std::min(batch, n - c);
             CTR_TRY(launch_adjoint_cols(*g, sino + (size_t)c * P, v0 + c, cnt, g->d_rays, vol, vdt,

@@ -16,7 +16,7 @@
 // voxel edge, or for rays nearly parallel to an axis.  Such irregular rays
 // (a few in 1e4) get a record of length 0 and mark their detector column;
 // the warps whose voxel columns see a marked detector column then visit its
-// irregular rays with the traversal's own cell intervals (AdjRay).  No
+// irregular rays with the traversal's own cell intervals (AdjIrr).  No
 // atomics; every sum has a fixed order.
 //
 // Bound by load latency and issue (half the slots): a row's records are loaded
@@ -30,10 +30,19 @@
 namespace ctr {
 
 // A ray's record: the detector value, and its length source - pixel; 0: no
-// chord; -0: an irregular ray, its traversal in the AdjRay array.
+// chord; -0: an irregular ray, its traversal in the AdjIrr array.
 struct __align__(8) AdjRec {
     float y, d12;
 };
+// An irregular ray: its length, the alphas it covers, its start voxel; the top
+// bit of i, j, k: parallel to the axis.  With the record 32 bytes a ray, as
+// k_adjoint's AdjRay, so that both kernels work on batches of the same views in
+// the same workspace.
+struct __align__(8) AdjIrr {
+    float d12, a_lo, a_hi;
+    int i, j, k;
+};
+static_assert(sizeof(AdjRec) + sizeof(AdjIrr) == sizeof(AdjRay), "one workspace for both adjoints");
 __device__ __forceinline__ bool irregular(const AdjRec& r) { return __float_as_uint(r.d12) == 0x80000000u; }
 
 // Records of views [view0, view0 + gridDim.z), [view][u][v].  A block of 32
@@ -42,7 +51,7 @@ __device__ __forceinline__ bool irregular(const AdjRec& r) { return __float_as_u
 static constexpr int AP_ROWS = 32, AP_COLS = 8;
 __global__ void __launch_bounds__(AP_ROWS * AP_COLS)
 k_adj_prep(const __grid_constant__ DevGeom g, const float* __restrict__ y, int view0, AdjRec* __restrict__ recs,
-           AdjRay* __restrict__ full, unsigned char* __restrict__ marks)
+           AdjIrr* __restrict__ full, unsigned char* __restrict__ marks)
 {
     __shared__ float yt[AP_COLS][AP_ROWS + 1];
     const int w = blockIdx.z, u0 = blockIdx.x * AP_COLS, v0 = blockIdx.y * AP_ROWS;
@@ -82,10 +91,9 @@ k_adj_prep(const __grid_constant__ DevGeom g, const float* __restrict__ y, int v
             const float INF = __int_as_float(0x7f800000);
             const RayResult rr = siddon<float, false, false, false>(g, g.px, g.py, g.pz, &INF, nullptr, sc.x, sc.y, u,
                                                                     v);
-            AdjRay a;
-            a.f = make_float4(yt[cu][rv], rr.d12, rr.a_lo, rr.a_hi);
-            a.i = make_int4(rr.vi0, rr.vj0, rr.vk0, rr.par);
-            full[w * P + (long long)u * g.ZP + v] = a;
+            auto axis = [&](int n, int bit) { return n | ((rr.par & bit) ? (int)0x80000000 : 0); };
+            full[w * P + (long long)u * g.ZP + v] =
+                AdjIrr{rr.d12, rr.a_lo, rr.a_hi, axis(rr.vi0, 1), axis(rr.vj0, 2), axis(rr.vk0, 4)};
             rec.d12 = -0.0f;
             marks[(long long)w * g.R + u] = 1;
         }
@@ -120,7 +128,7 @@ struct AdjWarp {
 
 // The irregular rays of the marked detector columns among a voxel column's candidates.
 static __device__ __noinline__ double irregular_sum(const DevGeom& g, const VoxCol& cc, int i, int j, int k, int view,
-                                                    const AdjRec* __restrict__ rw, const AdjRay* __restrict__ fw,
+                                                    const AdjRec* __restrict__ rw, const AdjIrr* __restrict__ fw,
                                                     const unsigned char* __restrict__ marks)
 {
     double acc = 0.0;
@@ -157,20 +165,22 @@ static __device__ __noinline__ double irregular_sum(const DevGeom& g, const VoxC
         const float ay0 = fm(fs(ylo, ct.z), ct.w), ay1 = fm(fs(yhi, ct.z), ct.w);
         for (int vv = vlo; vv <= vhi; ++vv) {
             const long long p = (long long)uu * g.ZP + vv;
-            if (!irregular(rw[p])) continue;
-            const AdjRay rec = fw[p];
+            const AdjRec rec = rw[p];
+            if (!irregular(rec)) continue;
+            const AdjIrr ray = fw[p];
+            const int ri = ray.i & 0x7fffffff, rj = ray.j & 0x7fffffff, rk = ray.k & 0x7fffffff;
             const float2 rt = g.rowt[vv];
             const float az0 = fm(fs(z0, rt.x), rt.y), az1 = fm(fs(z1, rt.x), rt.y);
             float xl, xh, yl, yh, zcl, zch;
-            if (!irregular_cell(i, rec.i.x, rec.i.w & 1, ax0, ax1, ct.y, xl, xh)) continue;
-            if (!irregular_cell(j, rec.i.y, rec.i.w & 2, ay0, ay1, ct.w, yl, yh)) continue;
-            if (!irregular_cell(k, rec.i.z, rec.i.w & 4, az0, az1, rt.y, zcl, zch)) continue;
-            const float lo = fmaxf(fmaxf(xl, yl), fmaxf(zcl, rec.f.z));
-            const float hi = fminf(fminf(xh, yh), fminf(zch, rec.f.w));
-            const float temp = fm(rec.f.y, fs(hi, lo));
-            const bool start = (i == rec.i.x) && (j == rec.i.y) && (k == rec.i.z);
+            if (!irregular_cell(i, ri, ray.i < 0, ax0, ax1, ct.y, xl, xh)) continue;
+            if (!irregular_cell(j, rj, ray.j < 0, ay0, ay1, ct.w, yl, yh)) continue;
+            if (!irregular_cell(k, rk, ray.k < 0, az0, az1, rt.y, zcl, zch)) continue;
+            const float lo = fmaxf(fmaxf(xl, yl), fmaxf(zcl, ray.a_lo));
+            const float hi = fminf(fminf(xh, yh), fminf(zch, ray.a_hi));
+            const float temp = fm(ray.d12, fs(hi, lo));
+            const bool start = (i == ri) && (j == rj) && (k == rk);
             // the traversal's first segment may be a rounding-size negative length
-            if (temp > 0.0f || (start && rec.f.z <= rec.f.w)) acc = __fma_rn((double)temp, (double)rec.f.x, acc);
+            if (temp > 0.0f || (start && ray.a_lo <= ray.a_hi)) acc = __fma_rn((double)temp, (double)rec.y, acc);
         }
     }
     return acc;
@@ -179,7 +189,7 @@ static __device__ __noinline__ double irregular_sum(const DevGeom& g, const VoxC
 template <typename VT>
 __global__ void __launch_bounds__(32 * AC_WARPS, 5)
 k_adj_cols(const __grid_constant__ DevGeom g, VT* __restrict__ vol, const AdjRec* __restrict__ recs,
-           const AdjRay* __restrict__ full, const unsigned char* __restrict__ marks, int view0, int nview, int accumulate)
+           const AdjIrr* __restrict__ full, const unsigned char* __restrict__ marks, int view0, int nview, int accumulate)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -292,7 +302,7 @@ k_adj_cols(const __grid_constant__ DevGeom g, VT* __restrict__ vol, const AdjRec
 size_t adj_record_bytes(const DevGeom& g, int views)
 {
     const size_t n = (size_t)g.R * g.ZP * views;
-    return n * (sizeof(AdjRec) + sizeof(AdjRay)) + (((size_t)g.R * views + 255) & ~(size_t)255);
+    return n * (sizeof(AdjRec) + sizeof(AdjIrr)) + (((size_t)g.R * views + 255) & ~(size_t)255);
 }
 
 ctr_status launch_adjoint_cols(const Geometry& G, const float* y, int view0, int nview, void* ws, void* vol,
@@ -301,8 +311,8 @@ ctr_status launch_adjoint_cols(const Geometry& G, const float* y, int view0, int
     const DevGeom& g = G.dg;
     if (nview <= 0) return CTR_OK;
     const size_t n = (size_t)g.R * g.ZP * nview;
-    AdjRay* full = (AdjRay*)ws;   // first: 16-byte aligned for any number of rays
-    AdjRec* recs = (AdjRec*)(full + n);
+    AdjIrr* full = (AdjIrr*)ws;
+    AdjRec* recs = (AdjRec*)(full + n);   // 8-byte aligned for any number of rays
     unsigned char* marks = (unsigned char*)(recs + n);
     CTR_CUDA_TRY(cudaMemsetAsync(marks, 0, (size_t)g.R * nview, st));
     k_adj_prep<<<dim3((g.R + AP_COLS - 1) / AP_COLS, (g.ZP + AP_ROWS - 1) / AP_ROWS, nview), AP_ROWS * AP_COLS, 0, st>>>(

@@ -49,3 +49,36 @@ def test_adjoint_tile_edges(name, oracle_built):
     half = torch.zeros(o.vol_shape, device="cuda", dtype=torch.bfloat16)
     g.backproject(dy, half)
     assert torch.equal(half.cpu(), torch.from_numpy(got.astype(np.float32)).to(torch.bfloat16))
+
+
+def test_adjoint_workspace_does_not_depend_on_the_call(oracle_built):
+    """The first call reserves a whole batch's ray records (about 256 MB at most), so a longer call neither allocates
+    nor moves them, and a captured short call can be replayed after it."""
+    import gpu_b200
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    cfg = scan(40, 36, 33, nu=512, nv=400, nviews=45, du=0.2)
+    g = gpu_b200.Geometry(ctr_desc(cfg))
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    y = torch.randn((45,) + g.view_shape, device="cuda", generator=gen)
+    long = torch.empty(g.vol_shape, device="cuda")
+    one = torch.empty(g.vol_shape, device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    g.backproject(y[7:8], one, 7, 1)
+    torch.cuda.synchronize()
+    first = torch.cuda.mem_get_info()[0]
+    assert before - first <= (256 << 20) + 512 * 64 * 8 + (4 << 20)   # records, marks, granularity
+    graph = torch.cuda.CUDAGraph()
+    out = torch.zeros_like(one)
+    with torch.cuda.graph(graph):
+        g.backproject(y[7:8], out, 7, 1)
+    torch.cuda.synchronize()
+    first = torch.cuda.mem_get_info()[0]
+    g.backproject(y, long)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == first   # (checked before the replay: it would use freed memory)
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, one)
