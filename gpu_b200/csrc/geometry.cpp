@@ -102,6 +102,16 @@ ctr_status ensure_tiled(Geometry* g, size_t bytes)
     return CTR_OK;
 }
 
+// While another thread captures a stream in the global mode (torch's default),
+// an allocation from this one, also a stream-ordered one, would invalidate that
+// capture.  Nothing of the pool is used by a captured stream, so its calls are
+// exempt.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // The geometry's pool, created by the first call that asks for it; nullptr where
 // the device has none.
 static cudaMemPool_t scratch_pool(Geometry* g)
@@ -130,6 +140,7 @@ void* pool_alloc(Geometry* g, size_t bytes, cudaStream_t st)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     void* p = nullptr;
     if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+        const RelaxedCapture relaxed;
         const cudaMemPool_t pool = scratch_pool(g);
         if (pool && cudaMallocFromPoolAsync(&p, bytes, pool, st) == cudaSuccess) return p;
     }
@@ -139,6 +150,7 @@ void* pool_alloc(Geometry* g, size_t bytes, cudaStream_t st)
 
 void pool_free(void* p, cudaStream_t st)
 {
+    const RelaxedCapture relaxed;
     if (p) cudaFreeAsync(p, st);
 }
 

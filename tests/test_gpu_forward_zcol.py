@@ -80,3 +80,43 @@ def test_zcol_forward_under_capture_and_on_streams():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(cap, want[0])
+
+
+def test_zcol_forward_beside_another_threads_capture():
+    """A call's scratch does not disturb a capture that another thread has open (in the global mode), neither the first
+    call of a geometry, which makes the pool, nor a later one."""
+    import threading
+
+    import gpu_b200
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    n = 10400
+    cfg = dict(widened(SMALL["cube16"]), nviews=n)
+    vol = torch.rand(gpu_b200.Geometry(ctr_desc(cfg)).vol_shape, device="cuda")
+    warm, new = (gpu_b200.Geometry(ctr_desc(cfg)) for _ in range(2))
+    side = torch.cuda.Stream()
+    outs = [torch.zeros((n,) + warm.view_shape, device="cuda") for _ in range(3)]
+    warm.forward(vol, outs[0])
+    torch.cuda.synchronize()
+    for g, out in ((warm, outs[1]), (new, outs[2])):
+        failed = []
+
+        def other():
+            try:
+                g.forward(vol, out, stream=side)
+            except Exception as e:
+                failed.append(e)
+
+        x = torch.zeros(64, device="cuda")
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, capture_error_mode="global"):
+            x += 1
+            t = threading.Thread(target=other)
+            t.start()
+            t.join()
+            x += 1
+        assert not failed
+        graph.replay()
+        torch.cuda.synchronize()
+        assert float(x.sum()) == 128.0
+        assert torch.equal(out, outs[0])
