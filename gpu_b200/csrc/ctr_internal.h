@@ -94,9 +94,10 @@ struct Geometry {
     void* d_tiled = nullptr; size_t tiled_bytes = 0;   // tiled copy for CTR_SART_TILED
     // Scratch of one call (ctr_forward's copy of the volume), stream-ordered, so
     // that calls on other streams and threads have their own.  The pool keeps
-    // at most about one FP32 volume between calls and goes with the geometry.
+    // pool_kept_bytes between calls and goes with the geometry.
     cudaMemPool_t pool = nullptr;
     bool pool_tried = false;
+    int rows_in = 0;                                   // detector rows of a view whose rays can meet the volume's height
     float* d_ramp = nullptr;                           // FDK's filter tables (fdk.cu): k_ramp_fft's, or 2R-1 taps
     // slab geometries of the one-GPU slab SART (ctr_sart_pass_slabs), built on first use,
     // with a stream per slab and the events that order them around the combination
@@ -139,6 +140,8 @@ ctr_status ensure_fgp(Geometry* g, size_t bytes);
 // FGP workspace: three sets of the three duals in the storage type
 inline size_t fgp_workspace_bytes(long long V, ctr_dtype dt) { return (size_t)V * 9 * dtype_size(dt); }
 ctr_status ensure_tiled(Geometry* g, size_t bytes);
+// what the geometry's pool keeps between calls: an FP32 volume and the pool's granularity
+inline size_t pool_kept_bytes(const Geometry& g) { return (size_t)g.nvox() * sizeof(float) + (64u << 20); }
 // bytes of the geometry's pool on stream st, or NULL (no memory, or st is being
 // captured: the caller then takes a path without scratch); pool_free returns it
 void* pool_alloc(Geometry* g, size_t bytes, cudaStream_t st);

@@ -125,7 +125,7 @@ static cudaMemPool_t scratch_pool(Geometry* g)
         pp.location.type = cudaMemLocationTypeDevice;
         pp.location.id = g->device;
         if (cudaMemPoolCreate(&g->pool, &pp) == cudaSuccess) {
-            uint64_t keep = (uint64_t)g->nvox() * sizeof(float) + (64u << 20);   // the pool's granularity
+            uint64_t keep = pool_kept_bytes(*g);
             cudaMemPoolSetAttribute(g->pool, cudaMemPoolAttrReleaseThreshold, &keep);
         } else {
             g->pool = nullptr;
@@ -433,12 +433,18 @@ static ctr_status create(const ctr_geometry_desc* din, int n_slabs, int slab, ct
         }
     }
     // BP row table: x1z and 1/(x2z-x1z) per detector row, same encoding.
+    // Rows that can meet the volume: at alpha a ray is at height x1z + alpha (x2z -
+    // x1z), and over the volume (its xy half-diagonal about the axis) alpha is in [a_lo, a_hi].
+    const double rv = 0.5 * std::hypot((double)d.nx * d.vx, (double)d.ny * d.vy) + std::fabs((double)d.m_offset * d.vx);
+    const double a_lo = (-rv - d.dod) / ((double)d.dso - d.dod), a_hi = (rv - d.dod) / ((double)d.dso - d.dod);
     std::vector<float2> rowt(q.ZP);
     for (int v = 0; v < q.ZP; ++v) {
         const int src = v / q.nvr, vr = v - src * q.nvr;
         const float x1z = q.zmin + (float)vr * q.dv;
         // fan slices, parallel beam: rows parallel to xy; tetrahedron beam: the band's source
         const float x2z = q.ct_style == 3 ? q.zsrc0 + (float)src * q.zsrc_dz : (q.ct_style == 0 ? q.srcz : x1z);
+        const double za = x1z + a_lo * ((double)x2z - x1z), zb = x1z + a_hi * ((double)x2z - x1z);
+        if (std::max(za, zb) >= q.bz && std::min(za, zb) <= (double)q.bz + (double)q.Z * q.vz) ++g->rows_in;
         if (std::fabs(x1z - x2z) < q.vz * 1e-6f) {
             const int kv = parallel_voxel(x1z, q.bz, q.inv_vz);
             rowt[v].x = plane(q.vz, kv, q.bz) + 0.5f * q.vz;

@@ -58,7 +58,13 @@ __host__ __device__ __forceinline__ int zcol_stride(const DevGeom& g, size_t es)
     const int q = 32 / (int)es;
     return (g.Z + q - 1) / q * q;
 }
-constexpr size_t ZF_SMEM_MOST = 200 * 1024;   // a list longer than this (one column) is left to the general projector
+constexpr size_t ZF_SMEM = 50 * 1024;   // of a block: four to an SM
+// Detector columns of a block: 4 (with 2 groups of 32 rows) while their lists fit
+// -- neighbouring columns cross the same voxel columns, and two warps share the
+// building of a list --, 2 with longer lists.  One column a block (above 3,060 x
+// and y planes) was never the faster path: 1600^2 x 64 voxels, 64 to 512 rows,
+// 125 to 14 ms against 27 to 13 ms.
+__host__ __forceinline__ int zf_columns(const DevGeom& g) { return zf_smem(g, 4) <= ZF_SMEM ? 4 : 2; }
 
 // The in-plane crossings of one detector column, in traversal order.
 struct Axis2 {
@@ -413,15 +419,11 @@ cudaError_t launch_zcol_t(const Geometry& G, const void* vol, const void* lin, i
 {
     const DevGeom& g = G.dg;
     const int zs = zcol_stride(g, sizeof(VT));
-    // 4 columns x 2 row groups a block while four blocks' lists fit an SM:
-    // neighbouring columns cross the same voxel columns, and two warps share
-    // the building of a list
-    int wc = 4;
-    while (wc > 1 && zf_smem(g, wc) > 50 * 1024) wc >>= 1;
+    const int wc = zf_columns(g);
     const void* fn = g.fast_sums ? reinterpret_cast<const void*>(&k_forward_zcol<VT, true>)
                                  : reinterpret_cast<const void*>(&k_forward_zcol<VT, false>);
     // one limit for every geometry: the attribute belongs to the function
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZF_SMEM_MOST);
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZF_SMEM);
     if (e != cudaSuccess) return e;
     const int per = 32 * (ZF_WARPS / wc);
     const dim3 grid((g.R + wc - 1) / wc, ((g.ct_style == 0 ? 2 * ((g.ZP + 1) / 2) : g.ZP) + per - 1) / per, nview);

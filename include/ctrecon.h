@@ -145,10 +145,11 @@ ctr_status ctr_geometry_autotune(ctr_geometry* geom, ctr_dtype vol_dtype, int n_
 /* sino[w] = A_(view_begin+w) vol for w < view_count (Siddon ray sums, command 0
  * of V63/kernel_IterativeRecon_universal.cu:7-567).  Replaces the per-view
  * launches of Forward_3D_ray_driven_siddon (V63/host_IterativeRecon_CBCT.c:70-128).
- * Large calls project a copy of vol in another layout, in stream-ordered scratch
- * of the call (about one volume, kept with the geometry between calls); without
- * the memory, or while the stream is captured, they project vol itself.  The
- * result is the same. */
+ * Large calls whose detector rows fill the other path's warps project a copy of
+ * vol in another layout, in stream-ordered scratch of the call (at most an FP32
+ * volume and 64 MiB, kept with the geometry between calls); without the memory,
+ * or while the stream is captured, they project vol itself.  The result is the
+ * same. */
 ctr_status ctr_forward(const ctr_geometry* geom, const void* vol, ctr_dtype vol_dtype,
                        void* sino, ctr_dtype sino_dtype, int view_begin, int view_count,
                        void* stream);

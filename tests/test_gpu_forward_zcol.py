@@ -2,12 +2,13 @@
 general projector (the same views one at a time, below that size), bit for bit:
 every scanner, odd and even detectors, exact 0/45/90-degree views (rays on
 planes, x and y planes crossed at one alpha), wide cones (rays entering and
-leaving through the z faces, several z planes a step), a volume touching the
-detector plane, offsets, the three storage types, fused sums, NaN voxels, and
+leaving through the z faces, several z planes a step), lists long enough for
+two columns a block, a volume touching the detector plane, offsets, the three storage types, fused sums, NaN voxels, and
 1 to 33 slices."""
 import numpy as np
 import pytest
 
+from kernels_run import kernels_run
 from scan_configs import NEAR_DETECTOR, SLABS, SMALL, STYLES, TBCT, ctr_desc, view_rows
 
 pytestmark = pytest.mark.gpu
@@ -17,16 +18,35 @@ LIST = dict(SMALL, near_detector=NEAR_DETECTOR, cone_wide=SLABS["cone_wide"], **
             square=dict(nx=20, ny=20, nz=9, nu=21, nv=7, nviews=8, vx=1.0, du=1.5, dso=1000.0, dod=-500.0, ct_style=2),
             flat=dict(nx=33, ny=17, nz=1, nu=40, nv=3, nviews=8, vx=1.0, du=1.2, dso=1000.0, dod=-500.0),
             tall=dict(nx=9, ny=40, nz=33, nu=41, nv=64, nviews=8, vx=1.0, du=1.0, dso=60.0, dod=-60.0),
+            long=dict(nx=850, ny=801, nz=24, nu=60, nv=24, nviews=8, vx=0.3, du=6.0, dso=1000.0, dod=-500.0),
             steep=dict(nx=8, ny=8, nz=64, nu=16, nv=70, nviews=8, vx=1.0, du=3.0, dso=30.0, dod=-30.0))
 
 
 # the path wants 480 x and y planes (900 for 16-bit voxels with the reference's
-# sums), 4.5e9 rays x planes and 120 a voxel: the scans' volumes are widened by more voxels of
-# a finer pitch, and the views repeat over many turns
+# sums), 4.5e9 rays x planes and 120 a voxel, and detector rows that fill its
+# blocks: the scans' volumes are widened by more voxels of a finer pitch, the
+# detector gets 127 or 128 rows over a little more than the volume's height
+# (the tetrahedron beam: sources for about 60 rows), and the views repeat over
+# many turns
 def widened(cfg):
     f = -(-900 // (cfg["nx"] + cfg["ny"]))
     nz = cfg["nz"] * f if "n_sources" in cfg else min(cfg["nz"] * f, 40)   # (the sources' places follow the height)
-    return dict(cfg, nx=cfg["nx"] * f, ny=cfg["ny"] * f, nz=nz, vx=cfg["vx"] / f, m_offset=cfg.get("m_offset", 0) * f)
+    out = dict(cfg, nx=cfg["nx"] * f, ny=cfg["ny"] * f, nz=nz, vx=cfg["vx"] / f, m_offset=cfg.get("m_offset", 0) * f)
+    if "n_sources" in cfg:
+        out["n_sources"] = {4: 16, 3: 21, 5: 11}[cfg["nv"]]
+    else:
+        cone = cfg.get("ct_style", 0) == 0
+        height = nz * (out["vx"] if cone else cfg["du"])
+        n = 128 - cfg["nv"] % 2
+        out.update(nv=n, dv=1.2 * height * ((cfg["dso"] - cfg["dod"]) / cfg["dso"] if cone else 1.0) / n)
+    return out
+
+
+def geometry(cfg, fast=False):
+    import gpu_b200
+    d = ctr_desc(cfg, fast_sums=fast)
+    d.dv = cfg.get("dv", 0.0)
+    return gpu_b200.Geometry(d)
 
 
 @pytest.mark.parametrize("fast", [False, True])
@@ -38,14 +58,19 @@ def test_zcol_equals_the_general_projector(name, fast):
     cfg = widened(LIST[name])
     rays = max(4.5e9, 120.0 * cfg["nx"] * cfg["ny"] * cfg["nz"]) / (cfg["nx"] + cfg["ny"])
     cfg["nviews"] = n = int(rays // (cfg["nu"] * view_rows(cfg)) // 8 + 1) * 8
-    g = gpu_b200.Geometry(ctr_desc(cfg, fast_sums=fast))
+    g = geometry(cfg, fast)
     gen = torch.Generator(device="cuda").manual_seed(4)
     base = torch.rand(g.vol_shape, device="cuda", generator=gen)
     base.view(-1)[base.numel() // 3] = float("nan")
     for dt in (torch.float32, torch.float16, torch.bfloat16):
         vol = base.to(dt)
         out = torch.zeros((n,) + g.view_shape, device="cuda")
-        g.forward(vol, out)
+        assert zcol_ran(lambda: g.forward(vol, out))
+        assert not zcol_ran(lambda: g.forward(vol, out[:1], 0, 1))
+        if dt != torch.float32:   # stored in 16 bits: the same sums rounded once
+            half = g.forward(vol, torch.zeros(out.shape, device="cuda", dtype=dt))
+            assert bool(((half == out.to(dt)) | (torch.isnan(half) & torch.isnan(out))).all())
+            del half
         one = torch.zeros((1,) + g.view_shape, device="cuda")
         for j in sorted({0, 1, n // 8, n // 4, n // 4 + 1, n // 2, 5 * n // 8, n - 1}):
             g.forward(vol, one, j, 1)
@@ -54,16 +79,39 @@ def test_zcol_equals_the_general_projector(name, fast):
             assert bool(same.all()), (j, dt, int((~same).sum()), float((out[j] - one[0]).abs().nan_to_num().max()))
 
 
+def zcol_ran(call):
+    names = kernels_run(call)
+    assert any("k_forward" in n for n in names), names
+    return any("k_forward_zcol" in n for n in names)
+
+
+def test_zcol_rule():
+    """Detector rows are the path's lanes, so rows that do not fill them, or do not meet the volume, keep the general
+    projector: (nx = ny, nz, nu, nv, taken)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    for n, nz, nu, nv, taken in ((512, 64, 1024, 64, True), (512, 32, 1024, 32, True), (512, 16, 1024, 16, False),
+                                 (512, 1, 2048, 1, False), (512, 4, 1024, 64, False), (512, 64, 1024, 72, False),
+                                 (512, 96, 1024, 96, True), (1024, 32, 512, 32, False), (1600, 64, 512, 256, False)):
+        views = int(max(4.6e9, 121.0 * n * n * nz) / (nu * nv * 2 * n)) + 1
+        g = geometry(dict(nx=n, ny=n, nz=nz, vx=256.0 / n, nu=nu, nv=nv, du=384.0 / nu,
+                          nviews=views, dso=1000.0, dod=-500.0, dv=384.0 / n))
+        vol = torch.rand(g.vol_shape, device="cuda")
+        out = torch.empty((views,) + g.view_shape, device="cuda")
+        assert zcol_ran(lambda: g.forward(vol, out)) == taken, (n, nz, nu, nv)
+
+
 def test_zcol_forward_under_capture_and_on_streams():
     """A captured call takes the path without scratch; calls on two streams have their own scratch."""
     import gpu_b200
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
-    n = 10400
+    n = 1640
     cfg = dict(widened(SMALL["cube16"]), nviews=n)
-    g = gpu_b200.Geometry(ctr_desc(cfg))
+    g = geometry(cfg)
     vols = [torch.rand(g.vol_shape, device="cuda") for _ in range(2)]
     want = [g.forward(v, torch.zeros((n,) + g.view_shape, device="cuda")) for v in vols]
+    assert zcol_ran(lambda: g.forward(vols[0], want[0]))
     torch.cuda.synchronize()
     outs = [torch.zeros_like(w) for w in want]
     streams = [torch.cuda.Stream() for _ in range(2)]
@@ -87,13 +135,12 @@ def test_zcol_forward_beside_another_threads_capture():
     call of a geometry, which makes the pool, nor a later one."""
     import threading
 
-    import gpu_b200
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
-    n = 10400
+    n = 1640
     cfg = dict(widened(SMALL["cube16"]), nviews=n)
-    vol = torch.rand(gpu_b200.Geometry(ctr_desc(cfg)).vol_shape, device="cuda")
-    warm, new = (gpu_b200.Geometry(ctr_desc(cfg)) for _ in range(2))
+    warm, new = (geometry(cfg) for _ in range(2))
+    vol = torch.rand(warm.vol_shape, device="cuda")
     side = torch.cuda.Stream()
     outs = [torch.zeros((n,) + warm.view_shape, device="cuda") for _ in range(3)]
     warm.forward(vol, outs[0])
