@@ -184,10 +184,7 @@ extern "C" ctr_status ctr_backproject(const ctr_geometry* geom, const float* sin
         if (!(flags & CTR_BP_ACCUMULATE)) CTR_CUDA_TRY(cudaMemsetAsync(vol, 0, g->nvox() * dtype_size(vdt), st));
         return CTR_OK;
     }
-    // The z-column gather reproduces the traversal of every scanner whose loop
-    // test is one comparison (no chord is cut short at the exit) with FP32
-    // entry; the other geometries and the masked form keep the general kernels.
-    if (!masked && g->dg.fast_exit && !g->dg.entry64 && g->dg.ct_style != 3) {
+    if (!masked && adjoint_cols_fits(*g)) {
         // for a whole batch whatever n is: the workspace of a captured call is not replaced by a longer one
         CTR_TRY(ensure_rays(g, adj_record_bytes(g->dg, batch)));
         for (int c = 0; c < n; c += batch) {

@@ -21,7 +21,7 @@
 // with the reference BP's geometric chords, FOV mask and thresholds.
 // k_adjoint: the exact adjoint of the forward projector, for the geometries the
 // z-column gather (zcol_adj.cu) does not cover (the tetrahedron beam, FP64 entry,
-// volumes that touch the detector plane).  Each ray record
+// volumes that touch the detector plane) or is slower for (few slices).  Each ray record
 // carries the alpha interval, start voxel and parallel axes of the forward
 // traversal, and the chord of a voxel is taken over the traversal's own cell
 // intervals: the start cell opens at -inf, cells behind the start are never
@@ -766,6 +766,11 @@ k_adjoint(const DevGeom g, VT* __restrict__ vol, const AdjRay* __restrict__ rays
 static size_t bp_smem(const DevGeom& g)
 {
     return sizeof(float) * (size_t)(g.M + 3 + g.N + 3 + ((g.Z + 3 + 1) & ~1)) + sizeof(float2) * g.ZP;
+}
+
+bool adjoint_tables_fit(const DevGeom& g)
+{
+    return std::max(bp_smem(g), sizeof(float) * (size_t)(g.M + g.N + g.Z + 16)) <= 48 * 1024;   // k_adjoint's, k_ray_prep's
 }
 
 // ------------------------------------------------- the batch's persistent pass

@@ -227,7 +227,9 @@ ctr_status forward_zcol(const Geometry& g, const void* vol, ctr_dtype vdt, void*
                         int view0, int nview, cudaStream_t st);
 // The matched adjoint as a z-column gather (zcol_adj.cu): views [view0,
 // view0 + nview) of y into vol.  ws: adj_record_bytes(g, nview) of scratch.
-// For fast_exit geometries with FP32 entry, the tetrahedron beam excepted.
+// For the geometries of adjoint_cols_fits; adjoint_tables_fit: k_adjoint's shared memory suffices.
+bool adjoint_cols_fits(const Geometry& g);
+bool adjoint_tables_fit(const DevGeom& g);
 size_t adj_record_bytes(const DevGeom& g, int views);
 ctr_status launch_adjoint_cols(const Geometry& g, const float* y, int view0, int nview, void* ws, void* vol,
                                ctr_dtype vdt, bool accumulate, cudaStream_t st);

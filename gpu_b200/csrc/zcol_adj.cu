@@ -102,7 +102,7 @@ k_adj_prep(const __grid_constant__ DevGeom g, const float* __restrict__ y, int v
 }
 
 static constexpr int AC_X = 8, AC_Y = 4, AC_N = AC_X * AC_Y;   // z-columns of a warp
-static constexpr int AC_WARPS = 4;                             // warps (z chunks of 32) of a block
+static constexpr int AC_WARPS = 4;                             // warps (z chunks of 32) of a block, at most
 
 // The chord of an irregular ray in voxel (i, j, k) over the traversal's own
 // cells: the start cell opens at -inf, cells behind the start are never
@@ -193,7 +193,7 @@ k_adj_cols(const __grid_constant__ DevGeom g, VT* __restrict__ vol, const AdjRec
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kb = (blockIdx.z * AC_WARPS + warp) * 32;
+    const int kb = (blockIdx.z * (blockDim.x >> 5) + warp) * 32;
     if (kb >= g.Z) return;   // no block-wide step below
     AdjWarp& W = reinterpret_cast<AdjWarp*>(smem_raw)[warp];
     const int i0 = blockIdx.x * AC_X, j0 = blockIdx.y * AC_Y;
@@ -305,6 +305,22 @@ size_t adj_record_bytes(const DevGeom& g, int views)
     return n * (sizeof(AdjRec) + sizeof(AdjIrr)) + (((size_t)g.R * views + 255) & ~(size_t)255);
 }
 
+// The gather reproduces the traversal of every scanner whose loop test is one
+// comparison (no chord is cut short at the exit) with FP32 entry, the tetrahedron
+// beam excepted; the others keep k_adjoint.  Its lanes are voxels of a z-column:
+// with few slices they idle, and k_adjoint, whose lanes run along x, is faster.
+// k_adjoint / here, ms, 32 views, 512^2 x nz voxels: cone beam (1.5 rows a voxel) nz = 1
+// 0.33 / 1.46, 4 1.30 / 1.97, 8 2.49 / 2.08, 16 4.60 / 2.13, 32 9.06 / 2.27; fan beam (1
+// row a voxel) nz = 1 0.33 / 1.45, 8 1.72 / 2.29, 16 3.11 / 2.34; parallel beam 8 1.45 /
+// 1.91, 16 2.65 / 1.93; the same lines at 192^2 to 1024^2.  (k_adjoint's tables are
+// in 48 KB of shared memory; without room for them the gather stays.)
+bool adjoint_cols_fits(const Geometry& G)
+{
+    const DevGeom& g = G.dg;
+    if (!g.fast_exit || g.entry64 || g.ct_style == 3) return false;
+    return g.Z >= (g.ct_style == 0 ? 8 : 12) || !adjoint_tables_fit(g);
+}
+
 ctr_status launch_adjoint_cols(const Geometry& G, const float* y, int view0, int nview, void* ws, void* vol,
                                ctr_dtype vdt, bool accumulate, cudaStream_t st)
 {
@@ -318,13 +334,16 @@ ctr_status launch_adjoint_cols(const Geometry& G, const float* y, int view0, int
     k_adj_prep<<<dim3((g.R + AP_COLS - 1) / AP_COLS, (g.ZP + AP_ROWS - 1) / AP_ROWS, nview), AP_ROWS * AP_COLS, 0, st>>>(
         g, y, view0, recs, full, marks);
     CTR_CUDA_TRY(cudaGetLastError());
-    const size_t smem = sizeof(AdjWarp) * AC_WARPS;
-    const int zc = (g.Z + 31) / 32;
-    const dim3 grid((g.M + AC_X - 1) / AC_X, (g.N + AC_Y - 1) / AC_Y, (zc + AC_WARPS - 1) / AC_WARPS);
+    // no more warps a block than there are z chunks for: an SM's 20 places go to
+    // working warps (512^2 x 32, 32 views: 2.27 ms; 5.27 with blocks of 4 warps)
+    const int zc = (g.Z + 31) / 32, gz = (zc + AC_WARPS - 1) / AC_WARPS, warps = (zc + gz - 1) / gz;
+    const size_t smem = sizeof(AdjWarp) * warps;
+    const dim3 grid((g.M + AC_X - 1) / AC_X, (g.N + AC_Y - 1) / AC_Y, gz);
     CTR_DISPATCH_DTYPE(vdt, VT, {
         CTR_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(&k_adj_cols<VT>),
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_adj_cols<VT><<<grid, 32 * AC_WARPS, smem, st>>>(g, (VT*)vol, recs, full, marks, view0, nview,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)(sizeof(AdjWarp) * AC_WARPS)));
+        k_adj_cols<VT><<<grid, 32 * warps, smem, st>>>(g, (VT*)vol, recs, full, marks, view0, nview,
                                                           accumulate ? 1 : 0);
     });
     CTR_CUDA_TRY(cudaGetLastError());

@@ -1,4 +1,4 @@
-"""The z-column adjoint at the edges of its tiles: volumes one voxel short of,
+"""The matched adjoint at the edges of the z-column gather's tiles and rule: volumes one voxel short of,
 at and past 8 x 4 columns and 32 slices, a single voxel, detector columns much
 finer than a voxel (runs longer than the four a column keeps) and coarser,
 steep cones, accumulation, 16-bit volumes.  Against the oracle's scatter of the
@@ -6,6 +6,7 @@ projector's own segments in FP64, to float rounding (as the parity test)."""
 import numpy as np
 import pytest
 
+from kernels_run import kernels_run
 from scan_configs import ctr_desc, og_desc_xyz
 
 pytestmark = pytest.mark.gpu
@@ -23,6 +24,10 @@ SCANS = {
     # an odd number of rays in a batch, axis-parallel and on-plane rays among them
     "odd_rays": scan(12, 12, 12, nu=17, nv=13, nviews=7, du=1.6),
     "odd_planes": scan(11, 12, 11, nu=17, nv=13, nviews=1, du=1.5),
+    # the slices at which the gather starts (7 / 8, fan and parallel beams 11 / 12), and warps of a block: 1, 2, 3 x 2
+    "7_slices": scan(34, 20, 7), "8_slices": scan(34, 20, 8), "11_fan": scan(33, 18, 11, ct_style=1),
+    "12_fan": scan(33, 18, 12, ct_style=1), "12_parallel": scan(33, 18, 12, ct_style=2), "40_slices": scan(9, 9, 40, nv=60),
+    "129_slices": scan(9, 5, 129, nv=90, du=2.0),
     "steep": scan(12, 10, 70, nu=24, nv=90, du=1.4, dso=30.0, dod=-30.0, initial_angle=3.0),
 }
 
@@ -39,7 +44,9 @@ def test_adjoint_tile_edges(name, oracle_built):
     ref = o.adjoint(y)
     dy = torch.from_numpy(y).cuda()
     vol = torch.full(o.vol_shape, 7.0, device="cuda")
-    g.backproject(dy, vol)                                     # overwrites
+    names = kernels_run(lambda: g.backproject(dy, vol))        # overwrites
+    gather = cfg["nz"] >= (12 if cfg.get("ct_style") else 8)
+    assert any("k_adj_cols" in n for n in names) == gather and any("k_adjoint" in n for n in names) != gather, names
     got = vol.cpu().numpy().astype(np.float64)
     top = np.abs(ref).max()
     assert top > 0
