@@ -54,7 +54,7 @@ struct RayInit {
     RayEnds e;
     float dx, dy, dz, ix, iy, iz;
     float amin, amax;       // entry and exit of the volume
-    float amin_xy;          // entry by the x and y faces alone
+    float a_last;           // exit by the faces of the axes the ray is not parallel to
     bool hit;               // amax > amin
     bool px, py, pz;        // parallel to the axis (the projector keeps its alpha infinite)
     AxisStart sx, sy, sz;   // at amin
@@ -72,7 +72,6 @@ __device__ __forceinline__ RayInit ray_init(const DevGeom& g, float s, float c, 
     const AxisSpan Zs = axis_span(__ldg(g.pz + 1), __ldg(g.pz + g.Z + 1), e.x1z, r.iz);
     r.amin = fmaxf(fmaxf(X.lo, Y.lo), fmaxf(Y.lo, Zs.lo));
     r.amax = fminf(fminf(X.hi, Y.hi), fminf(Y.hi, Zs.hi));
-    r.amin_xy = fmaxf(X.lo, Y.lo);
     r.hit = !(r.amax <= r.amin);
     r.px = fabsf(fs(e.x1x, e.x2x)) < fm(g.vx, 1e-6f);
     r.py = fabsf(fs(e.x1y, e.x2y)) < fm(g.vy, 1e-6f);
@@ -86,6 +85,7 @@ __device__ __forceinline__ RayInit ray_init(const DevGeom& g, float s, float c, 
         r.sz = axis_start(r.amin, Zs.lo, e.x1z, e.x2z, r.dz, g.bz, g.inv_vz, g.Z);
     }
     const float INF = __int_as_float(0x7f800000);
+    r.a_last = fminf(fminf(r.px ? INF : X.hi, r.py ? INF : Y.hi), r.pz ? INF : Zs.hi);
     r.ax = r.px ? INF : fm(fs(fa(fm(g.vx, (float)r.sx.plane), g.bx), e.x1x), r.ix);
     r.ay = r.py ? INF : fm(fs(fa(fm(g.vy, (float)r.sy.plane), g.by), e.x1y), r.iy);
     r.az = r.pz ? INF : fm(fs(fa(fm(g.vz, (float)r.sz.plane), g.bz), e.x1z), r.iz);

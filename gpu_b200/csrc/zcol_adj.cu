@@ -14,10 +14,11 @@
 // exactly the voxels with a positive overlap.  The reference's start rules
 // can miss it by one voxel when the entry lies within float rounding of a
 // voxel edge, or for rays nearly parallel to an axis.  Such irregular rays
-// (a few in 1e4) get a record of length 0 and mark their detector column;
-// the warps whose voxel columns see a marked detector column then visit its
-// irregular rays with the traversal's own cell intervals (AdjIrr).  No
-// atomics; every sum has a fixed order.
+// (a few in 1e4; at an axis-aligned view often whole rows and columns, whose
+// entries all lie on one plane) get a record of length 0 and set their row
+// group's bit in their detector column's mark; the warps whose voxel columns see
+// a marked detector column then visit those rays, a lane per column, with the
+// traversal's own cell intervals (AdjIrr).  Every sum has a fixed order.
 //
 // Bound by load latency and issue (half the slots): a row's records are loaded
 // a row ahead.  The form it replaces, which
@@ -45,13 +46,32 @@ struct __align__(8) AdjIrr {
 static_assert(sizeof(AdjRec) + sizeof(AdjIrr) == sizeof(AdjRay), "one workspace for both adjoints");
 __device__ __forceinline__ bool irregular(const AdjRec& r) { return __float_as_uint(r.d12) == 0x80000000u; }
 
+// A detector column's mark: bit b for irregular rays among rows [b << s, (b + 1) << s), s = mark_shift.
+typedef unsigned long long AdjMark;
+__host__ __device__ __forceinline__ int mark_shift(const DevGeom& g)
+{
+    int s = 0;
+    while (((g.ZP - 1) >> s) > 63) ++s;
+    return s;
+}
+__device__ __forceinline__ AdjMark mark_range(int vlo, int vhi, int s)   // the bits of rows vlo..vhi
+{
+    return (~0ull << (vlo >> s)) & (~0ull >> (63 - (vhi >> s)));
+}
+
+static __device__ __noinline__ float traversal_end(const DevGeom& g, float s, float c, int u, int v)
+{
+    const float INF = __int_as_float(0x7f800000);
+    return siddon<float, false, false, false>(g, g.px, g.py, g.pz, &INF, nullptr, s, c, u, v).a_hi;
+}
+
 // Records of views [view0, view0 + gridDim.z), [view][u][v].  A block of 32
 // columns x 8 rows; the records leave through shared memory so that the
 // transposed store is coalesced.
 static constexpr int AP_ROWS = 32, AP_COLS = 8;
 __global__ void __launch_bounds__(AP_ROWS * AP_COLS)
 k_adj_prep(const __grid_constant__ DevGeom g, const float* __restrict__ y, int view0, AdjRec* __restrict__ recs,
-           AdjIrr* __restrict__ full, unsigned char* __restrict__ marks)
+           AdjIrr* __restrict__ full, AdjMark* __restrict__ marks, int ms)
 {
     __shared__ float yt[AP_COLS][AP_ROWS + 1];
     const int w = blockIdx.z, u0 = blockIdx.x * AP_COLS, v0 = blockIdx.y * AP_ROWS;
@@ -88,14 +108,17 @@ k_adj_prep(const __grid_constant__ DevGeom g, const float* __restrict__ y, int v
         if (reg) {
             rec.d12 = ray_d12(r.e);
         } else if (ray_starts(g, r)) {
-            const float INF = __int_as_float(0x7f800000);
-            const RayResult rr = siddon<float, false, false, false>(g, g.px, g.py, g.pz, &INF, nullptr, sc.x, sc.y, u,
-                                                                    v);
-            auto axis = [&](int n, int bit) { return n | ((rr.par & bit) ? (int)0x80000000 : 0); };
+            // The traversal ends at the first plane alpha not below the exit, which is
+            // the exit itself -- the last plane of an axis the ray crosses -- unless a
+            // face the ray runs parallel to set it: such a ray is traversed (a view
+            // with one such ray waits for it, 0.1 ms at 96^3).
+            float a_hi = r.amax;
+            if (r.amax != r.a_last) a_hi = traversal_end(g, sc.x, sc.y, u, v);
+            auto axis = [&](int n, bool par) { return n | (par ? (int)0x80000000 : 0); };
             full[w * P + (long long)u * g.ZP + v] =
-                AdjIrr{rr.d12, rr.a_lo, rr.a_hi, axis(rr.vi0, 1), axis(rr.vj0, 2), axis(rr.vk0, 4)};
+                AdjIrr{ray_d12(r.e), r.amin, a_hi, axis(r.sx.v, r.px), axis(r.sy.v, r.py), axis(r.sz.v, r.pz)};
             rec.d12 = -0.0f;
-            marks[(long long)w * g.R + u] = 1;
+            atomicOr(marks + (long long)w * g.R + u, 1ull << (v >> ms));
         }
     }
     recs[w * P + (long long)u * g.ZP + v] = rec;
@@ -126,17 +149,10 @@ struct AdjWarp {
     VoxCol col[AC_N];
 };
 
-// The irregular rays of the marked detector columns among a voxel column's candidates.
-static __device__ __noinline__ double irregular_sum(const DevGeom& g, const VoxCol& cc, int i, int j, int k, int view,
-                                                    const AdjRec* __restrict__ rw, const AdjIrr* __restrict__ fw,
-                                                    const unsigned char* __restrict__ marks)
+// The magnifications of a voxel column's corners (the reference's rectangle): an
+// irregular ray's rows, to the nearest row.
+__device__ __forceinline__ float2 corner_mags(const DevGeom& g, int i, int j, int view)
 {
-    double acc = 0.0;
-    const float4* __restrict__ colt = g.colt + (long long)view * g.R;
-    const float xlo = __ldg(g.px + i + 1), xhi = __ldg(g.px + i + 2);
-    const float ylo = __ldg(g.py + j + 1), yhi = __ldg(g.py + j + 2);
-    const float z0 = __ldg(g.pz + k + 1), z1 = __ldg(g.pz + k + 2);
-    // rows from the corners' magnifications, to the nearest row (the reference's rectangle)
     const float2 sc = g.trig[view];
     const float cx = fa(fa(g.bx, fm(g.vx, 0.5f)), fm((float)i, g.vx));
     const float cy = fa(fa(g.by, fm(g.vy, 0.5f)), fm((float)j, g.vy));
@@ -149,47 +165,96 @@ static __device__ __noinline__ double irregular_sum(const DevGeom& g, const VoxC
         mlo = fminf(mlo, mt);
         mhi = fmaxf(mhi, mt);
     }
-    if (g.ct_style != 0) { mlo = 0.0f; mhi = 0.0f; }
-    const float zl = fs(z0, g.srcz), zh = fs(z1, g.srcz);
-    const float a0 = fa(fm(mlo, zl), z0), a1 = fa(fm(mhi, zl), z0), b0 = fa(fm(mlo, zh), z1), b1 = fa(fm(mhi, zh), z1);
-    const float zmn = fminf(fminf(a0, a1), fminf(b0, b1)), zmx = fmaxf(fmaxf(a0, a1), fmaxf(b0, b1));
-    int vlo = __float2int_rd(fa(fm(fs(zmn, g.zmin), g.inv_dv), 0.5f));
-    int vhi = __float2int_rd(fa(fm(fs(zmx, g.zmin), g.inv_dv), 0.5f));
-    if ((vlo < 0 && vhi < 0) || (vlo > g.ZP - 1 && vhi > g.ZP - 1)) return 0.0;
-    vlo = max(vlo, 0);
-    vhi = min(vhi, g.ZP - 1);
-    for (int uu = cc.ulo; uu <= cc.uhi; ++uu) {
-        if (!__ldg(marks + uu)) continue;
-        const float4 ct = __ldg(colt + uu);
-        const float ax0 = fm(fs(xlo, ct.x), ct.y), ax1 = fm(fs(xhi, ct.x), ct.y);
-        const float ay0 = fm(fs(ylo, ct.z), ct.w), ay1 = fm(fs(yhi, ct.z), ct.w);
-        for (int vv = vlo; vv <= vhi; ++vv) {
-            const long long p = (long long)uu * g.ZP + vv;
-            const AdjRec rec = rw[p];
-            if (!irregular(rec)) continue;
-            const AdjIrr ray = fw[p];
-            const int ri = ray.i & 0x7fffffff, rj = ray.j & 0x7fffffff, rk = ray.k & 0x7fffffff;
-            const float2 rt = g.rowt[vv];
-            const float az0 = fm(fs(z0, rt.x), rt.y), az1 = fm(fs(z1, rt.x), rt.y);
-            float xl, xh, yl, yh, zcl, zch;
-            if (!irregular_cell(i, ri, ray.i < 0, ax0, ax1, ct.y, xl, xh)) continue;
-            if (!irregular_cell(j, rj, ray.j < 0, ay0, ay1, ct.w, yl, yh)) continue;
-            if (!irregular_cell(k, rk, ray.k < 0, az0, az1, rt.y, zcl, zch)) continue;
-            const float lo = fmaxf(fmaxf(xl, yl), fmaxf(zcl, ray.a_lo));
-            const float hi = fminf(fminf(xh, yh), fminf(zch, ray.a_hi));
-            const float temp = fm(ray.d12, fs(hi, lo));
-            const bool start = (i == ri) && (j == rj) && (k == rk);
-            // the traversal's first segment may be a rounding-size negative length
-            if (temp > 0.0f || (start && ray.a_lo <= ray.a_hi)) acc = __fma_rn((double)temp, (double)rec.y, acc);
-        }
+    return g.ct_style != 0 ? make_float2(0.0f, 0.0f) : make_float2(mlo, mhi);
+}
+
+// The irregular rays that cross voxels kb .. kb + nk - 1 of the lane's voxel
+// column, into their sums acc[k - kb].  Called by the whole warp: every lane
+// finds its column's next ray, then those that have one work together.
+static __device__ __noinline__ void irregular_columns(const DevGeom& g, bool live, const VoxCol& cc, double* acc, int i, int j,
+                                                      int kb, int nk, int view, const AdjRec* __restrict__ rw,
+                                                      const AdjIrr* __restrict__ fw, const AdjMark* __restrict__ marks,
+                                                      int ms)
+{
+    const float4* __restrict__ colt = g.colt + (long long)view * g.R;
+    float xlo = 0.f, xhi = 0.f, ylo = 0.f, yhi = 0.f;
+    int vlo = 0, vhi = -1;
+    if (live) {
+        xlo = __ldg(g.px + i + 1); xhi = __ldg(g.px + i + 2);
+        ylo = __ldg(g.py + j + 1); yhi = __ldg(g.py + j + 2);
+        // candidate rows of the voxels together, to the nearest row
+        const float2 m = corner_mags(g, i, j, view);
+        const float z0 = __ldg(g.pz + kb + 1), z1 = __ldg(g.pz + kb + nk + 1);
+        const float zl = fs(z0, g.srcz), zh = fs(z1, g.srcz);
+        const float zmn = fminf(fa(fm(m.x, zl), z0), fa(fm(m.y, zl), z0));
+        const float zmx = fmaxf(fa(fm(m.x, zh), z1), fa(fm(m.y, zh), z1));
+        vlo = max(__float2int_rd(fa(fm(fs(zmn, g.zmin), g.inv_dv), 0.5f)), 0);
+        vhi = min(__float2int_rd(fa(fm(fs(zmx, g.zmin), g.inv_dv), 0.5f)), g.ZP - 1);
+        live = vlo <= vhi;
     }
-    return acc;
+    const AdjMark range = live ? mark_range(vlo, vhi, ms) : 0;
+    int uu = cc.ulo - 1, vv = 1, vend = 0;   // detector column; its rows of the current group left
+    AdjMark mark = 0;                        // its groups left
+    for (;;) {
+        bool found = false;
+        AdjRec rec;
+        while (live && !found) {
+            if (vv <= vend) {
+                rec = rw[(long long)uu * g.ZP + vv];
+                found = irregular(rec);
+                ++vv;
+            } else if (mark) {
+                const int g0 = (__ffsll(mark) - 1) << ms;
+                mark &= mark - 1;
+                vv = max(vlo, g0);
+                vend = min(vhi, g0 + (1 << ms) - 1);
+            } else if (uu < cc.uhi) {
+                mark = __ldg(marks + ++uu) & range;
+            } else {
+                live = false;
+            }
+        }
+        if (!__any_sync(0xffffffffu, found)) break;
+        if (found) {
+            const int v = vv - 1;
+            const AdjIrr ray = fw[(long long)uu * g.ZP + v];
+            const float2 rt = g.rowt[v];
+            const float4 ct = __ldg(colt + uu);
+            const float ax0 = fm(fs(xlo, ct.x), ct.y), ax1 = fm(fs(xhi, ct.x), ct.y);
+            const float ay0 = fm(fs(ylo, ct.z), ct.w), ay1 = fm(fs(yhi, ct.z), ct.w);
+            const int ri = ray.i & 0x7fffffff, rj = ray.j & 0x7fffffff, rk = ray.k & 0x7fffffff;
+            float xl, xh, yl, yh;
+            if (irregular_cell(i, ri, ray.i < 0, ax0, ax1, ct.y, xl, xh) &&
+                irregular_cell(j, rj, ray.j < 0, ay0, ay1, ct.w, yl, yh)) {
+                const float lo = fmaxf(fmaxf(xl, yl), ray.a_lo), hi = fminf(fminf(xh, yh), ray.a_hi);
+                // the voxels at the interval's two ends, a voxel of margin; the start voxel is the traversal's own
+                const float ka = ((rt.x + lo / rt.y) - g.bz) * g.inv_vz, kz = ((rt.x + hi / rt.y) - g.bz) * g.inv_vz;
+                int k0 = __float2int_rd(fminf(ka, kz)) - 1, k1 = __float2int_rd(fmaxf(ka, kz)) + 1;
+                const bool start_col = i == ri && j == rj;
+                if (start_col) {
+                    k0 = min(k0, rk);
+                    k1 = max(k1, rk);
+                }
+                for (int k = max(k0, kb); k <= min(k1, kb + nk - 1); ++k) {
+                    const float az0 = fm(fs(__ldg(g.pz + k + 1), rt.x), rt.y), az1 = fm(fs(__ldg(g.pz + k + 2), rt.x), rt.y);
+                    float zl, zh;
+                    if (!irregular_cell(k, rk, ray.k < 0, az0, az1, rt.y, zl, zh)) continue;
+                    const float temp = fm(ray.d12, fs(fminf(hi, zh), fmaxf(lo, zl)));
+                    // the traversal's first segment may be a rounding-size negative length
+                    if (temp > 0.0f || (start_col && k == rk && ray.a_lo <= ray.a_hi))
+                        acc[k - kb] = __fma_rn((double)temp, (double)rec.y, acc[k - kb]);
+                }
+            }
+        }
+        __syncwarp();
+    }
 }
 
 template <typename VT>
 __global__ void __launch_bounds__(32 * AC_WARPS, 5)
 k_adj_cols(const __grid_constant__ DevGeom g, VT* __restrict__ vol, const AdjRec* __restrict__ recs,
-           const AdjIrr* __restrict__ full, const unsigned char* __restrict__ marks, int view0, int nview, int accumulate)
+           const AdjIrr* __restrict__ full, const AdjMark* __restrict__ marks, int ms, int view0, int nview,
+           int accumulate)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -208,7 +273,7 @@ k_adj_cols(const __grid_constant__ DevGeom g, VT* __restrict__ vol, const AdjRec
     for (int w = 0; w < nview; ++w) {
         const int view = view0 + w;
         const AdjRec* __restrict__ rw = recs + w * P;
-        const unsigned char* __restrict__ mw = marks + (long long)w * g.R;
+        const AdjMark* __restrict__ mw = marks + (long long)w * g.R;
         __syncwarp();
         bool marked = false;
         {
@@ -279,11 +344,10 @@ k_adj_cols(const __grid_constant__ DevGeom g, VT* __restrict__ vol, const AdjRec
             }
             W.acc[q][lane] = acc;
         }
-        for (unsigned m = any_irr; m; m &= m - 1) {
-            const int q = __ffs(m) - 1;
-            if (k < g.Z)
-                W.acc[q][lane] += irregular_sum(g, W.col[q], i0 + (q % AC_X), j0 + q / AC_X, k, view, rw, full + w * P,
-                                                mw);
+        if (any_irr) {   // a lane per column again
+            __syncwarp();
+            irregular_columns(g, marked, W.col[lane], W.acc[lane], ci, cj, kb, min(32, g.Z - kb), view, rw, full + w * P, mw,
+                              ms);
         }
     }
     __syncwarp();
@@ -302,7 +366,7 @@ k_adj_cols(const __grid_constant__ DevGeom g, VT* __restrict__ vol, const AdjRec
 size_t adj_record_bytes(const DevGeom& g, int views)
 {
     const size_t n = (size_t)g.R * g.ZP * views;
-    return n * (sizeof(AdjRec) + sizeof(AdjIrr)) + (((size_t)g.R * views + 255) & ~(size_t)255);
+    return n * (sizeof(AdjRec) + sizeof(AdjIrr)) + (size_t)g.R * views * sizeof(AdjMark);
 }
 
 // The gather reproduces the traversal of every scanner whose loop test is one
@@ -329,10 +393,11 @@ ctr_status launch_adjoint_cols(const Geometry& G, const float* y, int view0, int
     const size_t n = (size_t)g.R * g.ZP * nview;
     AdjIrr* full = (AdjIrr*)ws;
     AdjRec* recs = (AdjRec*)(full + n);   // 8-byte aligned for any number of rays
-    unsigned char* marks = (unsigned char*)(recs + n);
-    CTR_CUDA_TRY(cudaMemsetAsync(marks, 0, (size_t)g.R * nview, st));
+    AdjMark* marks = (AdjMark*)(recs + n);
+    const int ms = mark_shift(g);
+    CTR_CUDA_TRY(cudaMemsetAsync(marks, 0, (size_t)g.R * nview * sizeof(AdjMark), st));
     k_adj_prep<<<dim3((g.R + AP_COLS - 1) / AP_COLS, (g.ZP + AP_ROWS - 1) / AP_ROWS, nview), AP_ROWS * AP_COLS, 0, st>>>(
-        g, y, view0, recs, full, marks);
+        g, y, view0, recs, full, marks, ms);
     CTR_CUDA_TRY(cudaGetLastError());
     // no more warps a block than there are z chunks for: an SM's 20 places go to
     // working warps (512^2 x 32, 32 views: 2.27 ms; 5.27 with blocks of 4 warps)
@@ -343,8 +408,8 @@ ctr_status launch_adjoint_cols(const Geometry& G, const float* y, int view0, int
         CTR_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(&k_adj_cols<VT>),
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)(sizeof(AdjWarp) * AC_WARPS)));
-        k_adj_cols<VT><<<grid, 32 * warps, smem, st>>>(g, (VT*)vol, recs, full, marks, view0, nview,
-                                                          accumulate ? 1 : 0);
+        k_adj_cols<VT><<<grid, 32 * warps, smem, st>>>(g, (VT*)vol, recs, full, marks, ms, view0, nview,
+                                                      accumulate ? 1 : 0);
     });
     CTR_CUDA_TRY(cudaGetLastError());
     return CTR_OK;

@@ -89,3 +89,26 @@ def test_adjoint_workspace_does_not_depend_on_the_call(oracle_built):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, one)
+
+
+@pytest.mark.parametrize("n", [96, 112])
+def test_adjoint_irregular_rays(n, oracle_built):
+    """An axis-aligned view where rays enter the volume within rounding of voxel edges (263 of 20,736 rays at 96^3, one
+    to three in most detector columns; 20 at 112^3), on more than 64 rows.  The traversal of such a ray may begin with a
+    segment as long as the rounding of its entry alpha, 2^-23 of the ray's length, which the gather leaves with the next
+    voxel: that, times the value, is the tolerance beside the regular rays' (test_adjoint_tile_edges)."""
+    import gpu_b200
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    p = 256.0 / n
+    cfg = scan(n, n, n, nu=n * 3 // 2, nv=n * 3 // 2, nviews=1, vx=p, du=p)
+    g = gpu_b200.Geometry(ctr_desc(cfg))
+    o = oracle_built.Oracle(og_desc_xyz(cfg))
+    y = np.random.default_rng(3).standard_normal((1,) + o.view_shape).astype(np.float32)
+    ref = o.adjoint(y)
+    vol = torch.zeros(o.vol_shape, device="cuda")
+    g.backproject(torch.from_numpy(y).cuda(), vol)
+    d12 = float(np.hypot(1500.0, 0.5 * cfg["nu"] * p * 2 ** 0.5))
+    err = np.abs(vol.cpu().numpy() - ref)
+    assert np.all(err <= 1.2e-7 * np.abs(ref) + 2.0 ** -23 * d12 * np.abs(y).max())
+    assert (err > 1.2e-7 * np.abs(ref) + 1e-12 * np.abs(ref).max()).sum() <= 1e-3 * ref.size
