@@ -278,10 +278,11 @@ k_forward_zcol(const __grid_constant__ DevGeom g, const VT* __restrict__ vol, in
             r.alim = t;
             if (sz) r.alim = fminf(r.alim, fm(fs(sz > 0 ? PZ[g.Z + 1] : PZ[1], in.e.x1z), in.iz));
             r.alim = fminf(r.alim, aend);
-            // at most one z crossing an entry: an entry is no longer than the step
-            // of either in-plane axis
-            ok = ok && fminf(g.vx, g.vy) > 1e-3f * g.vz &&
-                 fabsf(in.dz) * g.inv_vz < 0.999f * fmaxf(fabsf(in.dx) * g.inv_vx, fabsf(in.dy) * g.inv_vy);
+            // At most one z crossing an entry: an entry is no longer than the shorter
+            // in-plane step.  2^-20 for the rounding of the four alphas (below 4 x 2^-24
+            // each: the plane's subtraction, 1/d and the product, alphas below 1), 0.1 %
+            // for that of the planes' positions.
+            ok = ok && fminf(g.vx * fabsf(in.ix), g.vy * fabsf(in.iy)) * 1.001f + 9.5367432e-7f < g.vz * fabsf(in.iz);
             if (ok) {
                 r.live = ran = true;
                 r.n0 = n0;

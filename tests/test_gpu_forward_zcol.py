@@ -79,6 +79,27 @@ def test_zcol_equals_the_general_projector(name, fast):
             assert bool(same.all()), (j, dt, int((~same).sum()), float((out[j] - one[0]).abs().nan_to_num().max()))
 
 
+@pytest.mark.parametrize("fast", [False, True])
+def test_zcol_z_steps_as_short_as_in_plane_steps(fast):
+    """A cone so wide that a ray crosses about as many z planes as x or y planes, a thousand times magnified so that the
+    rounding of an alpha is a hundredth of a step: an entry of the list must not hold two z crossings."""
+    import gpu_b200
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    n, nz, nu = 240, 512, 128
+    views = int(4.6e9 // (2 * n * nu * nu)) + 1
+    mag = 1003.5 / 3.5
+    g = gpu_b200.Geometry(gpu_b200.make_desc(n, n, nz, 0.01, nu, nu, 1.2 * n * 0.01 * mag / nu, 3.5, -1000.0, views,
+                                             dv=1.2 * nz * 0.01 * mag / nu, fast_sums=fast))
+    vol = torch.rand(g.vol_shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    out = torch.zeros((views,) + g.view_shape, device="cuda")
+    one = torch.zeros((1,) + g.view_shape, device="cuda")
+    assert zcol_ran(lambda: g.forward(vol, out))
+    for j in range(0, views, 2):
+        g.forward(vol, one, j, 1)
+        assert torch.equal(out[j], one[0]), (j, int((out[j] != one[0]).sum()))
+
+
 def zcol_ran(call):
     names = kernels_run(call)
     assert any("k_forward" in n for n in names), names
