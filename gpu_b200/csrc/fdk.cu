@@ -15,6 +15,7 @@
 //      float/double steps, so the sum is the reference's to the bit).
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "ctr_device.cuh"
@@ -292,7 +293,7 @@ k_ramp_fft(const float* __restrict__ in, float* __restrict__ out, const FftTable
         }
 }
 
-static constexpr int FB_BX = 32, FB_BY = 4, FB_K = 8;
+static constexpr int FB_BX = 32, FB_BY = 4;
 
 // floor(x) and (int)floor(x) for 0 <= x < 2^22 without conversion
 // instructions (the backprojection is bound by the pipe that executes them):
@@ -326,15 +327,15 @@ template <bool RCP> __device__ __forceinline__ float div_by(float x, float d, fl
 
 // FULL: a full circle (us_rate*Nviews == 360).  Three divisions per voxel and
 // view (by the voxel column's distance, DSO and the row pitch) by div_by, what
-// does not depend on z once per FB_K voxels.  Bound by issue; 32 views into
+// does not depend on z once per K voxels of a column.  Bound by issue; 32 views into
 // 512^3: 7.3 ms (13.6 ms with IEEE divide sequences and 4 voxels a thread).
-template <bool FULL, bool RCP>
+template <bool FULL, bool RCP, int K>
 __global__ void __launch_bounds__(FB_BX * FB_BY)
 k_fdk_bp(const __grid_constant__ DevGeom g, float* __restrict__ vol, const float* __restrict__ proj, int view0, int nview)
 {
     const int i = blockIdx.x * FB_BX + (threadIdx.x % FB_BX);
     const int j = blockIdx.y * FB_BY + (threadIdx.x / FB_BX);
-    const int k0 = blockIdx.z * FB_K;
+    const int k0 = blockIdx.z * K;
     if (i >= g.M || j >= g.N) return;
     const long long MN = (long long)g.M * g.N;
     const int R = g.R, ZP = g.ZP;
@@ -343,9 +344,9 @@ k_fdk_bp(const __grid_constant__ DevGeom g, float* __restrict__ vol, const float
     // kernel_FDK.cu:86-88
     const float x = fa(fa(g.bx, fm(g.vx, 0.5f)), fm((float)i, g.vx));
     const float y = fa(fa(g.by, fm(g.vy, 0.5f)), fm((float)j, g.vy));
-    float acc[FB_K], dz[FB_K];
+    float acc[K], dz[K];
 #pragma unroll
-    for (int kk = 0; kk < FB_K; ++kk) {
+    for (int kk = 0; kk < K; ++kk) {
         const int k = min(k0 + kk, g.Z - 1);
         acc[kk] = vol[(long long)k * MN + (long long)j * g.M + i];
         dz[kk] = fm(DSO, fa(fa(g.bz, fm(g.vz, 0.5f)), fm((float)k, g.vz)));
@@ -364,7 +365,7 @@ k_fdk_bp(const __grid_constant__ DevGeom g, float* __restrict__ vol, const float
         const float bn0 = fs(p, floor_small(in_u ? p : 0.0f, bn)), bn1 = fs(1.0f, bn0);
         const float* __restrict__ pv = proj + (long long)w * R * ZP + bn;
 #pragma unroll
-        for (int kk = 0; kk < FB_K; ++kk) {
+        for (int kk = 0; kk < K; ++kk) {
             float ksi = div_by<RCP>(dz[kk], ds, r_ds);
             ksi = div_by<RCP>(fs(div_by<RCP>(fm(ksi, SDD), DSO, r_dso), g.zmin), g.dv, r_dv);
             float temp2 = 0.0f;
@@ -395,7 +396,7 @@ k_fdk_bp(const __grid_constant__ DevGeom g, float* __restrict__ vol, const float
         }
     }
 #pragma unroll
-    for (int kk = 0; kk < FB_K; ++kk) {
+    for (int kk = 0; kk < K; ++kk) {
         const int k = k0 + kk;
         if (k < g.Z) vol[(long long)k * MN + (long long)j * g.M + i] = acc[kk];
     }
@@ -567,7 +568,13 @@ ctr_status launch_fdk_bp(const Geometry& G, const float* fsino, int view0, int n
 {
     const DevGeom& g = G.dg;
     const long long P = G.npix();
-    dim3 grd((g.M + FB_BX - 1) / FB_BX, (g.N + FB_BY - 1) / FB_BY, (g.Z + FB_K - 1) / FB_K);
+    // 8 voxels a thread, or 4 while that leaves the GPU short of blocks (148 SMs x
+    // 4) and gives more of them.  4 / 8, ms, 180 views: 64^3 (256 blocks of 8) 0.326 /
+    // 0.417, 256^2 x 8 (512) 0.312 / 0.355, 64^2 x 4 0.213 / 0.196; above, 8 voxels share
+    // more of the in-plane work
+    const dim3 tiles((g.M + FB_BX - 1) / FB_BX, (g.N + FB_BY - 1) / FB_BY);
+    const bool wide = (long long)tiles.x * tiles.y * ((g.Z + 7) / 8) >= 148 * 4 || g.Z <= 4;
+    const dim3 grd(tiles.x, tiles.y, wide ? (g.Z + 7) / 8 : (g.Z + 3) / 4);
     // div_by: lengths far from the ends of the float range
     auto plain = [](float v) { return std::fabs(v) > 1e-9f && std::fabs(v) < 1e9f; };
     const bool rcp = plain(g.dso) && plain(g.dsod) && plain(g.du) && plain(g.dv) && plain(g.vx) && plain(g.vy) && plain(g.vz);
@@ -575,13 +582,17 @@ ctr_status launch_fdk_bp(const Geometry& G, const float* fsino, int view0, int n
     for (int w = 0; w < nview; w += VB) {
         const float* f = fsino + (size_t)P * w;
         const int n = std::min(VB, nview - w);
+        auto launch = [&](auto full, auto known) {
+            constexpr bool FULL = decltype(full)::value, RCP = decltype(known)::value;
+            if (wide) k_fdk_bp<FULL, RCP, 8><<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, f, view0 + w, n);
+            else k_fdk_bp<FULL, RCP, 4><<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, f, view0 + w, n);
+        };
         if (!rcp) {
-            if (g.fdk_full) k_fdk_bp<true, false><<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, f, view0 + w, n);
-            else k_fdk_bp<false, false><<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, f, view0 + w, n);
-        } else if (g.fdk_full) {
-            k_fdk_bp<true, true><<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, f, view0 + w, n);
+            if (g.fdk_full) launch(std::true_type(), std::false_type());
+            else launch(std::false_type(), std::false_type());
         } else {
-            k_fdk_bp<false, true><<<grd, FB_BX * FB_BY, 0, st>>>(g, vol, f, view0 + w, n);
+            if (g.fdk_full) launch(std::true_type(), std::true_type());
+            else launch(std::false_type(), std::true_type());
         }
     }
     CTR_CUDA_TRY(cudaGetLastError());

@@ -88,3 +88,28 @@ def test_fdk_smooth_rows(oracle_built):
     b = (5.0 + np.exp(-u ** 2) + 0.01 * np.cos(40 * u))[None, None, :] * (1.0 + 0.1 * np.arange(6))[None, :, None]
     got, want = both(cfg, o, np.repeat(b, 3, 0).astype(np.float32))
     assert np.abs(got - want).max() <= 1e-6 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("us", [360.0 / 3, 0.5])
+@pytest.mark.parametrize("shape", [(57, 148, 64), (61, 150, 40), (57, 144, 64), (7, 3, 33), (3, 5, 33), (1, 1, 1)])
+def test_fdk_backprojection_shapes(shape, us, oracle_built):
+    """The backprojection with 8 and with 4 voxels a thread (592 blocks of 8 and just below, few slices), a full circle
+    and a short scan, bit for bit against the reference kernel's arithmetic."""
+    import gpu_b200
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    nz, ny, nx = shape
+    cfg = dict(nx=nx, ny=ny, nz=nz, nu=90, nv=40, nviews=3, vx=1.0, du=2.0, dso=1000.0, dod=-500.0, initial_angle=2.0)
+    d = ctr_desc(cfg)
+    d.us_rate = us
+    od = og_desc_xyz(cfg)
+    od.us_rate = us
+    o = oracle_built.Oracle(od)
+    rng = np.random.default_rng(5)
+    filt = rng.standard_normal((3,) + o.view_shape).astype(np.float32)
+    want = rng.uniform(0, 1, o.vol_shape).astype(np.float32)
+    vol = torch.from_numpy(want.copy()).cuda()
+    gpu_b200.Geometry(d).fdk_backproject(torch.from_numpy(filt).cuda(), vol)
+    for j in range(3):
+        want = o.fdk_bp_view(want, filt[j], j)
+    assert np.array_equal(vol.cpu().numpy().view(np.uint32), np.asarray(want, np.float32).view(np.uint32))
