@@ -89,7 +89,8 @@ struct Geometry {
     void* d_rays = nullptr;  size_t rays_cap = 0;       // ray records (float2 SART / AdjRay adjoint)
     double* d_partial = nullptr; size_t partial_cap = 0;
     double* d_result = nullptr;                        // 8 doubles
-    void* d_fgp = nullptr; size_t fgp_bytes = 0;       // 9 dual arrays
+    void* d_fgp = nullptr; size_t fgp_bytes = 0;       // 9 dual arrays, or 6 and L (fgp.cu)
+    bool fgp_short = false;                            // the 9 did not fit the memory
     float* d_fdk = nullptr; size_t fdk_cap = 0;
     void* d_tiled = nullptr; size_t tiled_bytes = 0;   // tiled copy for CTR_SART_TILED
     // Scratch of one call (ctr_forward's copy of the volume), stream-ordered, so
@@ -137,8 +138,10 @@ inline bool dtype_ok(int t) { return t == CTR_F32 || t == CTR_BF16 || t == CTR_F
 ctr_status ensure_rays(Geometry* g, size_t bytes);
 ctr_status ensure_partial(Geometry* g, size_t n);
 ctr_status ensure_fgp(Geometry* g, size_t bytes);
-// FGP workspace: three sets of the three duals in the storage type
-inline size_t fgp_workspace_bytes(long long V, ctr_dtype dt) { return (size_t)V * 9 * dtype_size(dt); }
+// The FGP workspace for duals of type dt: three sets of the three duals, or, where
+// the one-pass iteration is not the faster one or its workspace does not fit, two
+// sets and L in FP32.
+ctr_status reserve_fgp(Geometry& g, ctr_dtype dt, bool* one_pass);
 ctr_status ensure_tiled(Geometry* g, size_t bytes);
 // what the geometry's pool keeps between calls: an FP32 volume and the pool's granularity
 inline size_t pool_kept_bytes(const Geometry& g) { return (size_t)g.nvox() * sizeof(float) + (64u << 20); }

@@ -3,12 +3,13 @@
 // FGP restates FGP_denoise_GPUx7_exact (V63/host_FGP_Denoise_GPUx7.c:1-111)
 // and its kernels FGP_operator_L_Pc / FGP_operator_LT_Pp
 // (V63/kernel_FGP_Denoise_GPUx7.cu:2-88) with the same float operations.  The
-// duals are stored in the volume's storage type; L is FP32 and never stored.
+// duals are stored in the volume's storage type; L is FP32.
 //
 // Dual layout: volume-sized arrays; r[p] belongs to the edge (x, x+1) and is 0
 // at x = nx-1 (the reference's zero-padded d_r[x+1], V63/host_FGP_Denoise_
 // GPUx7.c:8-38); likewise s along y and t along z.
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "ctr_device.cuh"
@@ -58,8 +59,8 @@ __device__ __forceinline__ float div_exact(float x, float d, float r)
 // formed from the two stored projections with the operations that stored it,
 // so r, s, t are never written: f and six arrays in, three out, 40 bytes a
 // voxel.  16-bit duals keep r, s, t as stored (their rounding differs from
-// one formed from the rounded o): 26 bytes a voxel.  The two-pass form (L
-// through HBM) moved 72 and 40 bytes.  An iteration: 512^3 FP32 1.25 ms
+// one formed from the rounded o): 24 bytes a voxel and f.  The two-pass form (L
+// through HBM) moves 72 and 40 bytes.  An iteration: 512^3 FP32 1.25 ms
 // (2.15 ms in two passes), 333x257x190 BF16 0.176 ms (0.245 ms).
 template <typename T> struct FgpSet {
     static constexpr bool REC = std::is_same<T, float>::value;
@@ -187,6 +188,53 @@ k_fgp_step(int M, int N, int Z, int zrun, const TF* __restrict__ f, const FgpSet
         for (int a = 0; a < 3; ++a) cur[a] = nxt[a];
         Lc = Ln;
     }
+}
+
+// One inner iteration in two passes, for volumes whose tiles k_fgp_step cannot
+// fill, and where its nine dual arrays do not fit the memory (one_pass): k_fgp_L
+// writes L for every voxel; k_fgp_dual reads L at the voxel and its +x, +y, +z
+// neighbours and updates the voxel's own six duals in place (no voxel reads
+// another's in this pass).  A thread a voxel, 32x8 tiles, no registers kept
+// between planes: twice the warps of k_fgp_step.  Bound by HBM and memory latency (2.6 to
+// 3.2 TB/s at 512^3), in L2 by latency.
+template <typename T, typename TF>
+__global__ void __launch_bounds__(FG_BX * FG_BY)
+k_fgp_L(int M, int N, int Z, const TF* __restrict__ f, const T* __restrict__ r, const T* __restrict__ s,
+        const T* __restrict__ t, float* __restrict__ L, float lambda)
+{
+    const int x = blockIdx.x * FG_BX + threadIdx.x, y = blockIdx.y * FG_BY + threadIdx.y, z = blockIdx.z;
+    if (x >= M || y >= N) return;
+    const long long MN = (long long)M * N, p = (long long)z * MN + (long long)y * M + x;
+    L[p] = fgp_L<T, TF>(f, r, s, t, x, y, z, p, M, MN, lambda);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(FG_BX * FG_BY)
+k_fgp_dual(int M, int N, int Z, const float* __restrict__ L, T* __restrict__ r, T* __restrict__ s, T* __restrict__ t,
+           T* __restrict__ o, T* __restrict__ pd, T* __restrict__ q, float alpha12, float gam)
+{
+    const int x = blockIdx.x * FG_BX + threadIdx.x, y = blockIdx.y * FG_BY + threadIdx.y, z = blockIdx.z;
+    if (x >= M || y >= N) return;
+    const long long MN = (long long)M * N, p = (long long)z * MN + (long long)y * M + x;
+    const bool e[3] = {x < M - 1, y < N - 1, z < Z - 1};
+    const long long up[3] = {1, M, MN};
+    T* const rst[3] = {r, s, t};
+    T* const old[3] = {o, pd, q};
+    const float Lc = __ldg(L + p);
+    float v[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        v[a] = Store<T>::ldw(rst[a] + p);
+        if (e[a]) v[a] = fa(v[a], fm(alpha12, fs(Lc, __ldg(L + p + up[a]))));
+    }
+    const float den = fmaxf(1.0f, __fsqrt_rn(fa(fa(fm(v[0], v[0]), fm(v[1], v[1])), fm(v[2], v[2]))));   // :78-86
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        if (e[a]) {
+            const float on = fdv(v[a], den);
+            Store<T>::st(rst[a] + p, fa(on, fm(gam, fs(on, Store<T>::ldw(old[a] + p)))));
+            Store<T>::st(old[a] + p, on);
+        }
 }
 
 // x* = f - lambda*div(o,p,q) (the final L_Pc, V63/host_FGP_Denoise_GPUx7.c:83);
@@ -319,14 +367,49 @@ static int grid_for(long long n, int threads)
 // t_k = (1 + sqrt(1 + 4 t^2))/2 in float (V63/host_FGP_Denoise_GPUx7.c:161)
 static float next_t(float t) { return (1.0f + sqrtf(1.0f + 4.0f * t * t)) / 2.0f; }
 
+// Whether the one-pass form is the faster one.  It needs tiles with work in them
+// (a third of the warps and more registers than the two-pass form), and planes to march
+// through; it gains most when the duals exceed the L2 cache, and halves the launches
+// of a volume that is little else (16^3 158 / 136).  Two passes / one, us
+// for 20 iterations: FP32 512x512x8 531 / 499, 2048x2048x1 1212 / 1434, x2 2725 / 2135,
+// 1024x1024x2 490 / 579, x3 953 / 783, 16x512x512 2315 / 1731, 8x512x512 1513 / 1651,
+// 512x9x512 719 / 819, 1024x2x1024 901 / 1264; BF16 2048x2048x1 840 / 1294, 16x512x512
+// 1629 / 1855, 20x512x512 1899 / 1893, 1024x4x1024 1159 / 1478, 33x512x512 4070 / 3268.
+static bool one_pass_faster(const Geometry& G, ctr_dtype dt)
+{
+    const double M = G.desc.nx, N = G.desc.ny, V = (double)G.nvox();
+    const double fill = M * N / (std::ceil(M / FG_BX) * FG_BX * std::ceil(N / FG_BY) * FG_BY);
+    const bool big = V * 9 * dtype_size(dt) > 100e6;
+    if (V <= 32768) return true;
+    if (big) return G.desc.nz >= 2 && fill >= 0.5;
+    return (G.desc.nz >= 3 || V <= 600e3) && fill >= 0.6;
+}
+
+ctr_status reserve_fgp(Geometry& G, ctr_dtype dt, bool* one_pass)
+{
+    const size_t V = (size_t)G.nvox(), es = dtype_size(dt), nine = 9 * es * V, seven = (6 * es + sizeof(float)) * V;
+    *one_pass = one_pass_faster(G, dt) && (G.fgp_bytes >= nine || !G.fgp_short);
+    if (*one_pass) {
+        const ctr_status r = ensure_fgp(&G, nine);
+        if (r != CTR_ERR_OUT_OF_MEMORY) return r;
+        clear_error();
+        cudaGetLastError();
+        G.fgp_short = true;   // (not tried again: every try would free and allocate)
+        *one_pass = false;
+    }
+    return ensure_fgp(&G, seven);
+}
+
 // The inner iterations of the prox of f: duals from zero, the last projections
-// o, p, q in D.  The geometry's workspace holds nine arrays of V duals.
+// o, p, q in D.  The geometry's workspace holds nine arrays of V duals, or six
+// and L.
 template <typename T, typename TF>
 static ctr_status fgp_iterations(Geometry& G, const TF* f, float lambda, int iters, T* D[3], cudaStream_t st)
 {
     const int M = G.desc.nx, N = G.desc.ny, Z = G.desc.nz;
     const long long V = G.nvox();
-    CTR_TRY(ensure_fgp(&G, fgp_workspace_bytes(V, DT<T>::v)));
+    bool one_pass;
+    CTR_TRY(reserve_fgp(G, DT<T>::v, &one_pass));
     T* base = (T*)G.d_fgp;
     T* A[3][3];   // [set][r s t]
     for (int i = 0; i < 3; ++i)
@@ -337,14 +420,28 @@ static ctr_status fgp_iterations(Geometry& G, const TF* f, float lambda, int ite
         return CTR_OK;
     }
     const float alpha12 = 1.0f / (lambda * 12.0f);                 // :166
+    float t_k_1 = 1.0f, gam_prev = 0.0f;
+    if (!one_pass) {   // o, p, q in set 0, r, s, t in set 1, then L
+        float* L = (float*)((char*)G.d_fgp + 6 * (size_t)V * sizeof(T));
+        const dim3 blk(FG_BX, FG_BY), grd((M + FG_BX - 1) / FG_BX, (N + FG_BY - 1) / FG_BY, Z);
+        CTR_CUDA_TRY(cudaMemsetAsync(base, 0, 6 * (size_t)V * sizeof(T), st));
+        for (int it = 0; it < iters; ++it) {
+            const float t_k = next_t(t_k_1);
+            k_fgp_L<T, TF><<<grd, blk, 0, st>>>(M, N, Z, f, A[1][0], A[1][1], A[1][2], L, lambda);
+            k_fgp_dual<T><<<grd, blk, 0, st>>>(M, N, Z, L, A[1][0], A[1][1], A[1][2], A[0][0], A[0][1], A[0][2], alpha12,
+                                               (t_k_1 - 1.0f) / t_k);
+            t_k_1 = t_k;
+        }
+        CTR_CUDA_TRY(cudaGetLastError());
+        return CTR_OK;
+    }
     // z planes per block: long runs (each recomputes one plane of L) while the
-    // blocks still fill the GPU about three times (148 SMs x 4 blocks)
+    // blocks still fill the GPU six times (148 SMs x 4 blocks)
     const long long tiles = (long long)((M + FG_BX - 1) / FG_BX) * ((N + FG_BY - 1) / FG_BY);
     int zrun = 32;
     while (zrun > 4 && tiles * ((Z + zrun - 1) / zrun) < 148LL * 24) zrun >>= 1;
     zrun = std::max(zrun, (Z + 65534) / 65535);
     const dim3 blk(32, FG_BY + 1), grd((M + FG_BX - 1) / FG_BX, (N + FG_BY - 1) / FG_BY, (Z + zrun - 1) / zrun);
-    float t_k_1 = 1.0f, gam_prev = 0.0f;
     for (int it = 0; it < iters; ++it) {
         const float t_k = next_t(t_k_1);
         const float gam = (t_k_1 - 1.0f) / t_k;
@@ -411,7 +508,8 @@ ctr_status launch_refine_update(Geometry& G, float* xk, float* xm, const void* d
     const long long V = G.nvox();
     const bool fgp = lam > 0.f && iters >= 0;
     if (ddt != dt && ddt != CTR_F32) return set_error(CTR_ERR_INVALID_ARGUMENT, "correction type");
-    if (fgp) CTR_TRY(ensure_fgp(&G, fgp_workspace_bytes(V, dt)));
+    bool one_pass;
+    if (fgp) CTR_TRY(reserve_fgp(G, dt, &one_pass));   // before xm is written over
     const int nb = grid_for(V, 256);
     CTR_DISPATCH_DTYPE(dt, T, {
         if (ddt == CTR_F32) k_refine_sum<T, float><<<nb, 256, 0, st>>>(G.dg, xk, xm, (const float*)d_tiled, gdev);

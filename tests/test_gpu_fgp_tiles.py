@@ -6,6 +6,8 @@ numpy, the duals rounded to the storage type (FP32 and FP16) after each step
 import numpy as np
 import pytest
 
+from kernels_run import kernels_run
+
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 F = np.float32
@@ -76,3 +78,74 @@ def test_fgp_block_edges(shape, dtype):
         want = prox(vol, lam, iters, dt)
         got = x.cpu().numpy()
         assert np.array_equal(got, want), (lam, iters, np.abs(got.astype(F) - want.astype(F)).max())
+
+
+def run(shape, dtype, lam_iters, form):
+    import gpu_b200
+    nz, ny, nx = shape
+    dt = {"f32": np.float32, "f16": np.float16}[dtype]
+    g = gpu_b200.Geometry(gpu_b200.make_desc(nx, ny, nz, 0.1, 16, 16, 1.0, 1000.0, -1000.0, 4))
+    rng = np.random.default_rng(nx + 100 * ny)
+    vol = (rng.uniform(0, 0.05, shape) + 0.2 * (rng.random(shape) > 0.9)).astype(dt)
+    names = kernels_run(lambda: g.fgp_tv(torch.from_numpy(vol.copy()).cuda(), 0.01, 2))
+    assert any("k_fgp_step" in n for n in names) == (form == "one pass"), names
+    assert any("k_fgp_dual" in n for n in names) == (form == "two passes"), names
+    for lam, iters in lam_iters:
+        x = torch.from_numpy(vol.copy()).cuda()
+        g.fgp_tv(x, lam, iters)
+        want = prox(vol, lam, iters, dt)
+        assert np.array_equal(x.cpu().numpy(), want), (lam, iters)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("shape,form", [
+    # one pass: full tiles, a voxel short of and past them, runs of 4 planes and remainders
+    ((4, 8, 32), "one pass"), ((9, 16, 65), "one pass"), ((35, 15, 63), "one pass"), ((5, 25, 64), "one pass"),
+    ((33, 33, 97), "one pass"), ((2, 40, 96), "one pass"), ((1, 7, 31), "one pass"), ((6, 9, 33), "one pass"),
+    # two: tiles mostly empty
+    ((33, 33, 33), "two passes"), ((40, 1, 900), "two passes"), ((90, 80, 5), "two passes"), ((40, 9, 129), "two passes")])
+def test_fgp_forms(shape, form, dtype):
+    """The one-pass and the two-pass iteration, each where the rule takes it."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    run(shape, dtype, ((0.01, 1), (0.01, 2), (0.01, 5), (1e-4, 3)), form)
+
+
+@pytest.mark.parametrize("shape,dtype,form", [((1, 1024, 1024), "f32", "two passes"), ((2, 1024, 1024), "f16", "two passes"),
+                                              ((2, 1300, 1300), "f32", "one pass"), ((400, 504, 16), "f32", "one pass"),
+                                              ((400, 504, 16), "f16", "two passes")])
+def test_fgp_forms_large(shape, dtype, form):
+    """Few planes and half-filled tiles, on both sides of the size at which the duals exceed the L2 cache."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    run(shape, dtype, ((0.01, 2),), form)
+
+
+def test_fgp_in_short_memory():
+    """Where nine dual arrays do not fit the memory the prox runs in two passes on six and L: the same bits."""
+    import gpu_b200
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    n = (256, 512, 512)
+    desc = gpu_b200.make_desc(n[2], n[1], n[0], 0.1, 16, 16, 1.0, 1000.0, -1000.0, 4)
+    vol = torch.rand(n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    g = gpu_b200.Geometry(desc)
+    want = g.fgp_tv(vol.clone(), 0.01, 3)
+    g.close()
+    got = vol.clone()
+    g = gpu_b200.Geometry(desc)
+    # the two-pass kernels are loaded before the memory is taken
+    gpu_b200.Geometry(gpu_b200.make_desc(1024, 1024, 1, 0.1, 16, 16, 1.0, 1000.0, -1000.0, 4)).fgp_tv(
+        torch.rand((1, 1024, 1024), device="cuda"), 0.01, 1)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    V = vol.numel()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - 32 * V, dtype=torch.uint8, device="cuda")   # between 28 V and 36 V left
+    try:
+        g.fgp_tv(got, 0.01, 3)
+        assert torch.equal(got, want)
+        names = kernels_run(lambda: g.fgp_tv(got, 0.01, 1))
+        assert any("k_fgp_dual" in k for k in names) and not any("k_fgp_step" in k for k in names), names
+    finally:
+        del hold
+        torch.cuda.empty_cache()
