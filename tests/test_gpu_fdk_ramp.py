@@ -1,8 +1,9 @@
 """FDK's ramp filter at the row lengths where its FFT changes shape: the
 smallest, those around a power of two (2R-1 points at least: one more point
 doubles the transform), every last radix (8, 4, 2), an odd number of rows, and
-rows too long for the FFT (the Toeplitz product).  Against the oracle's FDK
-(FP64 taps, direct sums) within 1e-4 of its maximum, as the FDK parity test."""
+rows too long for the FFT (the Toeplitz product).  The voxels read the rows
+from end to end, where a transform one point short would show.  Against the
+oracle's FDK (FP64 taps, direct sums rounded to FP32)."""
 import numpy as np
 import pytest
 
@@ -12,23 +13,35 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-@pytest.mark.parametrize("nu", [4, 5, 16, 17, 32, 33, 64, 65, 100, 4096, 4097])
+@pytest.mark.parametrize("nu", [4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 100, 500, 1024, 1025, 4096, 4097])
 def test_fdk_row_lengths(nu, oracle_built):
+    """One slice as wide as the detector sees, so that every column is read.  Random rows: the filter's FP32 rounding and
+    the backprojection's, 2e-6 of the largest voxel (1e-5 for the Toeplitz product's 4097 FP32 terms).  Impulses at both
+    ends of a row, one view: the far columns hold the taps of the longest lags, 1e-3 to 1e-7 of the largest, each to
+    some ten FP32 roundings of itself."""
     import gpu_b200
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
-    cfg = dict(nx=10, ny=10, nz=6, nu=nu, nv=7, nviews=3, vx=1.0, du=1.6, dso=1000.0, dod=-500.0)
-    if nu > 1000:
-        cfg.update(nv=5, nviews=1, nz=2)
-    g = gpu_b200.Geometry(ctr_desc(cfg))
-    d = og_desc_xyz(cfg)
-    o = oracle_built.Oracle(d)
-    b = np.random.default_rng(nu).standard_normal((cfg["nviews"],) + o.view_shape).astype(np.float32)
-    vol = torch.zeros(o.vol_shape, device="cuda")
-    g.fdk(torch.from_numpy(b).cuda(), vol)
-    ref = o.fdk(b)
-    assert np.abs(ref).max() > 0
-    assert np.abs(vol.cpu().numpy() - ref).max() <= 1e-4 * np.abs(ref).max()
+    n = max(10, min(nu, 200))
+    cfg = dict(nx=n, ny=n, nz=1, nu=nu, nv=7, nviews=3, vx=200.0 / n, du=1.5 * 200.0 / nu, dso=1000.0, dod=-500.0)
+
+    def both(cfg, b):
+        o = oracle_built.Oracle(og_desc_xyz(cfg))
+        vol = torch.zeros(o.vol_shape, device="cuda")
+        gpu_b200.Geometry(ctr_desc(cfg)).fdk(torch.from_numpy(b).cuda(), vol)
+        return vol.cpu().numpy(), o.fdk(b)
+
+    got, ref = both(cfg, np.random.default_rng(nu).standard_normal((3, 7, nu)).astype(np.float32))
+    top = np.abs(ref).max()
+    assert top > 0 and np.abs(got - ref).max() <= (2e-6 if nu <= 4096 else 1e-5) * top
+    for at in (0, nu - 1):
+        b = np.zeros((1, 7, nu), np.float32)
+        b[:, :, at] = 1.0
+        got, ref = both(dict(cfg, nviews=1), b)
+        err, mag = np.abs(got - ref), np.abs(ref)
+        far = mag <= 1e-3 * mag.max()
+        assert mag.max() > 0 and np.all(err <= 1e-6 * mag.max())
+        assert np.all(err[far] <= 1e-6 * mag[far] + 1e-12 * mag.max())
 
 
 def rows_scan(nu, nv):
