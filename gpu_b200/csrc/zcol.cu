@@ -53,8 +53,8 @@ static bool zf_rows_fill(const Geometry& G)
 // * a call pays for its lists and copy, and the first one maps the scratch
 //   (0.9 ms for 37 MB, 3.7 ms for 512 MB), which it should win back: 4.5e9 steps,
 //   and 120 a voxel.  426x424x288, 5 views (1.1e9) 0.93 / 0.83; 301x259x211, 60
-//   views (4.2e9) 2.95 / 3.10; 256^3, 64 views (4.8e9) 3.39 / 4.61; 512^3, 32
-//   views (2.6e10) 15.8 / 24.5;
+//   views (4.2e9) 2.95 / 3.10, but a first call 3.95 / 3.17; 256^3, 64 views
+//   (4.8e9) 3.39 / 4.61; 512^3, 32 views (2.6e10) 15.8 / 24.5;
 // * short rays do not repay a list: 480 x and y planes (200x180x150, 60 views
 //   1.12 / 1.06);
 // * with 16-bit voxels and the reference's sums a step converts two voxels and

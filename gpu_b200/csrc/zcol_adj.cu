@@ -20,11 +20,11 @@
 // a marked detector column then visit those rays, a lane per column, with the
 // traversal's own cell intervals (AdjIrr).  Every sum has a fixed order.
 //
-// Bound by load latency and issue (half the slots): a row's records are loaded
-// a row ahead.  The form it replaces, which
-// tested every candidate pair against the traversal record in 32 bytes, took
-// 0.59 ms a view of 256^3 voxels and 384^2 rays, records included; this one
-// takes 0.14 ms (0.15 with 16-byte records and no load ahead).
+// Bound by issue and load latency (60 % of the issue slots): a row's records are
+// loaded a row ahead.  The form it replaces, which tested every candidate pair
+// against the traversal record in 32 bytes, takes 0.60 ms a view of 256^3 voxels
+// and 384^2 rays, records included; this one 0.13 ms (0.15 with 16-byte records
+// and no load ahead).
 #include "fp_kernels.cuh"
 #include "zcol_bp.cuh"
 

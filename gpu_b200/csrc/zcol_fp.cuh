@@ -24,14 +24,14 @@
 // first crossing does not lie after its entry (the start rules' rounding), is
 // walked by the general projector (zf_general).
 //
-// Bound by issue (78 % of the slots, 440 M instructions a view of 512^3 and
+// Bound by issue (80 % of the slots, 446 M instructions a view of 512^3 and
 // 1024 x 768 rays): a step takes about 27 instructions, a third of them for the
 // z crossing that any of a warp's rows may make; the general kernel takes about
 // 40 (three plane alphas re-evaluated each step).  In the cone beam the two
 // halves of a warp take rows mirrored about the middle row: mirrored rays cross
-// z planes at the same steps.  Per view, copy included, over 8 views: FP32
-// 0.55 ms (general kernel on the linear volume 0.78 ms), BF16 0.54 (0.86), fused
-// sums 0.50 and 0.49 (0.78 and 0.86).
+// z planes at the same steps.  Per view, copy included, over 32 views at 35 to 46
+// degrees: FP32 0.59 ms (general kernel on the linear volume 0.84 ms), BF16 0.59
+// (0.92), fused sums 0.54 and 0.55 (0.83 and 0.92).
 #pragma once
 
 #include "fp_kernels.cuh"
