@@ -1,18 +1,21 @@
 """The names of the kernels that a call launches, from the profiler's activity
-records.  The profiler now and then drops a short kernel's record, so the call
-is made three times, and again if nothing was recorded."""
+records.  The profiler can drop records, so a kernel that is absent here may
+have run; one that is present did."""
+import time
+
 import torch
 
 
 def kernels_run(call):
-    names = set()
-    for _ in range(4):
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
+        time.sleep(0.02)
+        for _ in range(3):
+            call()
         torch.cuda.synchronize()
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
-            for _ in range(3):
-                call()
-            torch.cuda.synchronize()
-        names |= {e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA}
-        if names:
-            break
-    return sorted(names)
+        time.sleep(0.02)
+    return sorted({e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA})
+
+
+def none_of(names, *kernels):
+    return not any(k in n for n in names for k in kernels)
