@@ -106,7 +106,8 @@ k_ramp(const float* __restrict__ in, float* __restrict__ out, const float* __res
 // k_fdk_weight's operations, zero beyond R); the inverse's first pass separates
 // the two interleaved spectra, multiplies by the taps' spectrum (real: the taps
 // are even) and joins them again; its last pass writes the row.  Short rows
-// share a block.
+// share a block.  The length is a template parameter: with the passes unrolled and
+// their addresses folded a row of 1024 takes 60 % of the time.
 //
 // FP64 because the ramp removes what a smooth row is made of, low frequencies:
 // an FP32 transform's error follows the row's largest values and is several
@@ -115,12 +116,11 @@ k_ramp(const float* __restrict__ in, float* __restrict__ out, const float* __res
 // row with a non-finite value is summed directly (its transform would turn one
 // Inf into NaN everywhere), with k_ramp's operations.
 //
-// Bound by latency and shared memory (8 exchanges of 16 KB for 1024 values),
-// 24 warps an SM (78 registers).  256 views x 768 rows of 1024: 4.0 ms, weight
-// included; 4.4 ms at 16 warps; FP32 pairs of rows 3.2 ms; the Toeplitz product
-// and the weight pass 10.4 ms.  64 rows of 64, 360 views: 45, 52 and 63 us.
+// Bound by shared memory (8 exchanges of 16 KB for 1024 values; the LSU data pipe
+// at 92 %), 24 warps an SM.  256 views x 768 rows of 1024: 2.34 ms, weight
+// included (4.0 ms with the length as an argument); FP32 pairs of rows 3.10 ms; the
+// Toeplitz product and the weight pass 10.3 ms.  360 x 64 rows of 64: 15, 31 and 27 us.
 static constexpr int kFftMost = 8192;     // 512 threads, 74 KB of shared memory
-static constexpr int kFftBlock = 128;     // threads of a block of short rows
 
 __device__ __forceinline__ int fft_pad(int i) { return i + (i >> 3); }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
@@ -191,16 +191,17 @@ __device__ __forceinline__ void fft_radix(double2* v, int j, int ns, int n, cons
 // between the points go through sh.  The forward's get does not read sh, the
 // inverse's put does not write it.  The sub-transform lengths are 1, 8, 64, ...; a
 // last pass of radix 2 or 4 does 4 or 2 butterflies a thread.
-template <bool INV, typename G, typename P>
-__device__ __forceinline__ void fft_passes(double2* sh, int j, int n, int log2n, const double2* __restrict__ tw, G get, P put)
+template <bool INV, int LOG2N, typename G, typename P>
+__device__ __forceinline__ void fft_passes(double2* sh, int j, const double2* __restrict__ tw, G get, P put)
 {
-    const int T = n >> 3;
+    constexpr int n = 1 << LOG2N, T = n >> 3;
     double2 v[8];
-    int ns = 1;
-    for (int left = log2n; left > 0;) {
-        const bool first = ns == 1;
-        const int lr = left >= 3 ? 3 : left;
-        const bool last = left == lr;
+#pragma unroll
+    for (int done = 0; done < LOG2N; done += 3) {   // levels of the transform
+        const int ns = 1 << done;
+        const bool first = done == 0;
+        const int lr = min(3, LOG2N - done);
+        const bool last = done + lr == LOG2N;
         const bool reads = INV || !first, writes = !INV || !last;   // of sh
         if (reads) __syncthreads();   // the previous pass's stores
         if (lr == 3) {
@@ -228,8 +229,6 @@ __device__ __forceinline__ void fft_passes(double2* sh, int j, int n, int log2n,
             if (last) put(at, v[q]);
             else sh[fft_pad(at)] = v[q];
         }
-        ns <<= lr;
-        left -= lr;
     }
 }
 
@@ -243,17 +242,20 @@ struct FftTables {
     const float* taps;
 };
 
-// Rows of nrows rows of R values (row % ZP is the detector row): out = ramp(weight
-// * in).  A block takes blockDim.x / (N/8) rows.
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == kFftBlock ? 6 : 1)
+// nrows rows of R values (row % ZP is the detector row): out = ramp(weight * in).
+// A block takes fft_rows rows of N/8 threads.
+constexpr int fft_rows(int log2N) { return log2N < 10 ? 1024 >> log2N : 1; }
+constexpr int fft_threads(int log2N) { return fft_rows(log2N) << (log2N - 3); }   // 128, 256, 512
+template <int LOG2N>
+__global__ void __launch_bounds__(fft_threads(LOG2N), 6 * 128 / fft_threads(LOG2N))
 k_ramp_fft(const float* __restrict__ in, float* __restrict__ out, const FftTables tb, float dso, int R, int ZP,
-           long long nrows, int N, int log2N)
+           long long nrows)
 {
+    constexpr int N = 1 << LOG2N, T = N >> 3;
     extern __shared__ double2 fsh[];
-    __shared__ int bad[kFftBlock];   // rows with a non-finite value
-    const int T = N >> 3, rl = threadIdx.x / T, j = threadIdx.x - rl * T;
-    const long long row = (long long)blockIdx.x * (blockDim.x / T) + rl;
+    __shared__ int bad[fft_rows(LOG2N)];   // rows with a non-finite value
+    const int rl = threadIdx.x / T, j = threadIdx.x % T;
+    const long long row = (long long)blockIdx.x * fft_rows(LOG2N) + rl;
     const bool live = row < nrows;
     double2* const sh = fsh + (size_t)rl * (N + T);
     const float* __restrict__ a = in + (live ? row : 0) * R;
@@ -262,7 +264,7 @@ k_ramp_fft(const float* __restrict__ in, float* __restrict__ out, const FftTable
     __syncthreads();
     auto value = [&](int i) { return fdv(fm(__ldg(a + i), dso), __ldg(rt + i)); };   // kernel_FDK.cu:1-14
     bool off = false;
-    fft_passes<false>(sh, j, N, log2N, tb.tw, [&](int i) {
+    fft_passes<false, LOG2N>(sh, j, tb.tw, [&](int i) {
         float x = 0.0f, y = 0.0f;
         if (live && 2 * i < R) x = value(2 * i);
         if (live && 2 * i + 1 < R) y = value(2 * i + 1);
@@ -273,7 +275,7 @@ k_ramp_fft(const float* __restrict__ in, float* __restrict__ out, const FftTable
     // Z = E + iO, the spectra of the even and the odd points; with the taps'
     // X[k] = E + W O, X[k+N] = E - W O become H[k] X[k], H[N-k] X[k+N]
     float* __restrict__ o = out + (live ? row : 0) * R;
-    fft_passes<true>(sh, j, N, log2N, tb.tw, [&](int k) {
+    fft_passes<true, LOG2N>(sh, j, tb.tw, [&](int k) {
         const double2 z = sh[fft_pad(k)], y = sh[fft_pad((N - k) & (N - 1))];
         const double2 w = __ldg(tb.un + 2 * k), h = __ldg(tb.un + 2 * k + 1);
         const double2 e = make_double2(0.5 * (z.x + y.x), 0.5 * (z.y - y.y));
@@ -516,19 +518,32 @@ ctr_status launch_fdk(Geometry& G, const float* sino, float* vol, cudaStream_t s
     float* fsino = G.d_fdk;
     const long long nrows = (long long)nv * g.ZP;
     if (fft) {
-        const int N = (int)(n / 2), T = N / 8, rows = std::max(1, kFftBlock / T);   // rows of a block
-        int log2N = 0;
-        while ((1 << log2N) < N) ++log2N;
-        const size_t smem = (size_t)rows * (N + T) * sizeof(double2);
-        const unsigned blocks = (unsigned)((nrows + rows - 1) / rows);
+        const size_t N = n / 2;
         const FftTables tb = fft_table_pointers(G, N);
-        if (rows * T == kFftBlock) {
-            k_ramp_fft<kFftBlock><<<blocks, kFftBlock, smem, st>>>(sino, fsino, tb, g.dso, g.R, g.ZP, nrows, N, log2N);
-        } else {
-            CTR_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(&k_ramp_fft<kFftMost / 16>),
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
-            k_ramp_fft<kFftMost / 16><<<blocks, rows * T, smem, st>>>(sino, fsino, tb, g.dso, g.R, g.ZP, nrows, N, log2N);
+        auto launch = [&](auto log2N) -> cudaError_t {
+            constexpr int L = decltype(log2N)::value, rows = fft_rows(L);
+            constexpr size_t smem = (size_t)rows * ((1 << L) + (1 << L >> 3)) * sizeof(double2);
+            const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&k_ramp_fft<L>),
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+            k_ramp_fft<L><<<(unsigned)((nrows + rows - 1) / rows), fft_threads(L), smem, st>>>(sino, fsino, tb, g.dso, g.R,
+                                                                                             g.ZP, nrows);
+            return cudaGetLastError();
+        };
+        cudaError_t e = cudaErrorInvalidValue;
+        switch (N) {
+        case 8: e = launch(std::integral_constant<int, 3>()); break;
+        case 16: e = launch(std::integral_constant<int, 4>()); break;
+        case 32: e = launch(std::integral_constant<int, 5>()); break;
+        case 64: e = launch(std::integral_constant<int, 6>()); break;
+        case 128: e = launch(std::integral_constant<int, 7>()); break;
+        case 256: e = launch(std::integral_constant<int, 8>()); break;
+        case 512: e = launch(std::integral_constant<int, 9>()); break;
+        case 1024: e = launch(std::integral_constant<int, 10>()); break;
+        case 2048: e = launch(std::integral_constant<int, 11>()); break;
+        case 4096: e = launch(std::integral_constant<int, 12>()); break;
         }
+        CTR_CUDA_TRY(e);
     } else {
         float* wsino = G.d_fdk + (size_t)P * nv;
         for (int v0 = 0; v0 < nv; v0 += 65535) {
